@@ -268,9 +268,10 @@ int mt_qgemm_rope_append(void* stream, const void* x, const uint32_t* qweight, c
  *   offsets_dev (device int32 [batch], may be NULL) gives every sequence its own offset_b, else `offset` holds for all.
  *   fp32 throughout, one rounding (the tensor-core kernels, d == 64 or 128, multiply the probabilities as the sum of two
  *   16-bit terms).  mt_rope_append (any even d) fills the cache of one sequence at a time.
- * mt_attention_batch: the same with a workspace of at least mt_attention_batch_workspace_bytes(m, hq, hkv, d), zeroed once by
- *   the caller (the kernels leave its counters zeroed; word 0 is the error word): up to 16 query rows per kv head
- *   (m * hq / hkv) then run on a kernel that streams the caches once, split evenly over the GPU whatever the lengths.
+ * mt_attention_batch: the same with a workspace of at least mt_attention_batch_workspace_bytes(m, hq, hkv, d) (0: the request
+ *   uses none): up to 16 query rows per kv head (m * hq / hkv) then run on a kernel that streams the caches once, split
+ *   evenly over the GPU whatever the lengths.  The workspace belongs to the call until it has run and may hold anything
+ *   before (the call zeroes what it counts in, on its stream).  Word 0 is the error word, written only when a wait expired.
  */
 int mt_attention(void* stream, const void* q, const void* k_cache, const void* v_cache, void* out, const int32_t* offsets_dev,
                  int batch, int m, int hq, int hkv, int d, int offset, int capacity, float scale, int dtype);

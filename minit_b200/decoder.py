@@ -105,17 +105,6 @@ def qkv_rope_append(x: torch.Tensor, qweight: torch.Tensor, zeros: Optional[torc
 
 
 _att_ws = _lib.attention_workspaces
-_batch_ws = {}
-
-
-def _zeroed_workspace(table, dev: torch.device, stream: int, need: int) -> torch.Tensor:
-    """One workspace per (device, stream), zeroed once: the attention kernels leave their counters zeroed."""
-    key = (dev.index, stream)
-    ws = table.get(key)
-    if ws is None or ws.numel() < need:
-        ws = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=dev)
-        table[key] = ws
-    return ws
 
 
 def attention_decode(q: torch.Tensor, cache: KVCache, offset: int, offset_dev: Optional[torch.Tensor] = None,
@@ -131,7 +120,11 @@ def attention_decode(q: torch.Tensor, cache: KVCache, offset: int, offset_dev: O
     max_len = cache.capacity if offset_dev is not None else offset + m
     need = _lib.lib.mt_attention_workspace_bytes(m, cache.kv_heads, max_len)
     stream = _lib.current_stream(dev)
-    ws = _zeroed_workspace(_att_ws, dev, stream, need)
+    key = (dev.index, stream)
+    ws = _att_ws.get(key)
+    if ws is None or ws.numel() < need:
+        ws = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=dev)       # zeroed once; the kernel leaves it zeroed
+        _att_ws[key] = ws
     if out is None:
         out = torch.empty((m, hq * d), dtype=q.dtype, device=dev)
     with torch.cuda.device(dev):
@@ -162,11 +155,13 @@ def attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, off
         raise ValueError("offsets must be int32 [B]")
     if out is None:
         out = torch.empty((b, m, hq * d), dtype=q.dtype, device=dev)
-    stream = _lib.current_stream(dev)
-    ws = _zeroed_workspace(_batch_ws, dev, stream, _lib.lib.mt_attention_batch_workspace_bytes(m, hq, hkv, d))
+    need = _lib.lib.mt_attention_batch_workspace_bytes(m, hq, hkv, d)
+    # scratch of this call alone (the caching allocator's, 3 MB at most): graphs that are captured on one stream, and replayed
+    # in any order or on several streams, share nothing
+    ws = torch.empty(need, dtype=torch.uint8, device=dev) if need else None
     with torch.cuda.device(dev):
-        rc = _lib.lib.mt_attention_batch(stream, q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), _lib.ptr(offsets),
-                                         b, m, hq, hkv, d, offset, capacity, 1.0 / math.sqrt(d), ws.data_ptr(), ws.numel(),
+        rc = _lib.lib.mt_attention_batch(_lib.current_stream(dev), q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(),
+                                         _lib.ptr(offsets), b, m, hq, hkv, d, offset, capacity, 1.0 / math.sqrt(d), _lib.ptr(ws), need,
                                          _lib.dtype_code(q.dtype))
     _lib.check(rc, "mt_attention_batch")
     return out
