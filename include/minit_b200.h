@@ -272,6 +272,8 @@ int mt_qgemm_rope_append(void* stream, const void* x, const uint32_t* qweight, c
  *   uses none): up to 16 query rows per kv head (m * hq / hkv) then run on a kernel that streams the caches once, split
  *   evenly over the GPU whatever the lengths.  The workspace belongs to the call until it has run and may hold anything
  *   before (the call zeroes what it counts in, on its stream).  Word 0 is the error word, written only when a wait expired.
+ * mt_attention_error: the current device's error word of both (0, or 8: a bounded wait expired since it was last cleared and
+ *   the outputs of the calls in between are not valid).  Copies from the device: call it after the stream was synchronised.
  */
 int mt_attention(void* stream, const void* q, const void* k_cache, const void* v_cache, void* out, const int32_t* offsets_dev,
                  int batch, int m, int hq, int hkv, int d, int offset, int capacity, float scale, int dtype);
@@ -279,6 +281,7 @@ size_t mt_attention_batch_workspace_bytes(int m, int hq, int hkv, int d);
 int mt_attention_batch(void* stream, const void* q, const void* k_cache, const void* v_cache, void* out, const int32_t* offsets_dev,
                        int batch, int m, int hq, int hkv, int d, int offset, int capacity, float scale,
                        void* workspace, size_t workspace_bytes, int dtype);
+int mt_attention_error(uint32_t* word, int clear);
 size_t mt_attention_workspace_bytes(int m, int hkv, int max_len);
 int mt_attention_decode(void* stream, const void* q, const void* k_cache, const void* v_cache, void* out, int m, int hq, int hkv, int d,
                         int offset, const int32_t* offset_dev, int max_len, float scale, void* workspace, size_t workspace_bytes, int dtype);

@@ -65,6 +65,7 @@ SYMBOLS = {
     "mt_attention": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, ctypes.c_float, _i]),
     "mt_attention_batch_workspace_bytes": (_sz, [_i, _i, _i, _i]),
     "mt_attention_batch": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, ctypes.c_float, _vp, _sz, _i]),
+    "mt_attention_error": (_i, [ctypes.POINTER(ctypes.c_uint32), _i]),
     "mt_attention_workspace_bytes": (_sz, [_i, _i, _i]),
     "mt_attention_decode": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp, _i, ctypes.c_float, _vp, _sz, _i]),
     "mt_decode_plan": (_i, [_i, _i, _i, _i, _i, _sz, _i]),
@@ -158,8 +159,20 @@ def workspace_error_word(ws: torch.Tensor) -> int:
     return int(ws[COUNTER_BYTES - 4:COUNTER_BYTES].view(torch.int32).item())
 
 
+attention_devices = set()       # indices of the devices that ran decoder.attention: their error word is in the library, not in a workspace
+
+
+def attention_error_word(device: int, clear: bool) -> int:
+    """Error word of decoder.attention on one device (8: a bounded wait expired).  Synchronises with the current stream."""
+    word = ctypes.c_uint32(0)
+    with torch.cuda.device(device):
+        torch.cuda.current_stream().synchronize()
+        check(lib.mt_attention_error(ctypes.byref(word), int(clear)), "mt_attention_error")
+    return word.value
+
+
 def raise_on_error_words(clear: bool = True) -> None:
-    """Check the error word of every workspace of this process and raise ``MinitError`` (status
+    """Check the error word of every workspace of this process, and of every device that ran ``decoder.attention``, and raise ``MinitError`` (status
     ``ERR_PEER_TIMEOUT``) if a bounded device-side wait expired since the last check: the outputs of the
     calls in between are not valid (after an expired all-reduce wait the ranks no longer hold the same
     values).  It reads device memory, so call it where the host synchronises anyway -- after the read-back
@@ -171,6 +184,10 @@ def raise_on_error_words(clear: bool = True) -> None:
             bad.append((key, word))
             if clear:
                 ws[COUNTER_BYTES - 4:COUNTER_BYTES].zero_()
+    for device in attention_devices:
+        word = attention_error_word(device, clear)
+        if word:
+            bad.append(((device, "attention"), word))
     if bad:
         err = MinitError(ERR_PEER_TIMEOUT, "bounded device-side wait")
         err.words = bad

@@ -537,6 +537,12 @@ int mt_attention_batch(void* stream, const void* q, const void* k_cache, const v
     return launch_attention_rows(st, q, k_cache, v_cache, out, offsets_dev, batch, m, hq, hkv, d, offset, capacity, scale, dtype);
 }
 
+int mt_attention_error(uint32_t* word, int clear) {
+    if (!word) return MT_ERR_NULL;
+    const int rc = check_device();
+    return rc != MT_OK ? rc : attention_error(word, clear != 0);
+}
+
 int mt_attention(void* stream, const void* q, const void* k_cache, const void* v_cache, void* out, const int32_t* offsets_dev,
                  int batch, int m, int hq, int hkv, int d, int offset, int capacity, float scale, int dtype) {
     return mt_attention_batch(stream, q, k_cache, v_cache, out, offsets_dev, batch, m, hq, hkv, d, offset, capacity, scale, nullptr, 0, dtype);

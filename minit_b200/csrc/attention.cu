@@ -49,6 +49,10 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t&
     else lo = H::pack(a - H::to_float(uint16_t(hi & 0xffff)), b - H::to_float(uint16_t(hi >> 16)));
 }
 
+// Set to 8 by a kernel of this file whose wait ran out, read by mt_attention_error.  One word per device, in the module itself: calls
+// without a workspace and calls whose scratch is gone by the time the host looks report here too.
+__device__ unsigned g_attention_error;
+
 // On a wait that ran out: give the copies in flight time to land before the shared memory is given up.
 __device__ __forceinline__ void drain_copies() { for (int i = 0; i < 1000; ++i) __nanosleep(1000); }
 
@@ -415,7 +419,10 @@ attention_stream_kernel(const __grid_constant__ CUtensorMap mk, const __grid_con
     }
     griddep_wait();                                                 // in every CTA: this grid never ends before the zeroing one
     __syncthreads();
-    if (tid == 0 && s_abort && p.ws) *reinterpret_cast<unsigned*>(p.ws) = 8u;
+    if (tid == 0 && s_abort) {
+        g_attention_error = 8u;
+        *reinterpret_cast<unsigned*>(p.ws) = 8u;
+    }
 }
 
 // ------------------------------------------------------------------------------------------------------------
@@ -686,7 +693,10 @@ attention_tile_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
     tc_fence_before();
     __syncthreads();
     if (warp == 0) { tc_fence_after(); tc_dealloc<512>(tmem); }
-    if (tid == 0 && s_abort && p.err) *p.err = 8u;
+    if (tid == 0 && s_abort) {
+        g_attention_error = 8u;
+        if (p.err) *p.err = 8u;
+    }
 }
 
 // q / out [batch, m, heads, d] (heads = hq) or a cache [batch, capacity, hkv, d] as (64 d, rows.., halves ..) boxes of a
@@ -754,6 +764,15 @@ bool attention_batch_supported(int hq, int hkv, int d) { return (d == 64 || d ==
 size_t attention_batch_workspace_bytes(int m, int hq, int hkv, int d) {
     if (m < 1 || hq < 1 || !attention_batch_supported(hq, hkv, d) || (long long)m * (hq / hkv) > 16) return 0;      // no scratch
     return AS_PART_OFF + (size_t)AS_GRID * 2 * 16 * (d + 4) * 4;
+}
+
+int attention_error(unsigned* word, bool clear) {
+    unsigned w = 0;
+    const unsigned zero = 0;
+    if (cudaMemcpyFromSymbol(&w, g_attention_error, 4) != cudaSuccess ||
+        (w && clear && cudaMemcpyToSymbol(g_attention_error, &zero, 4) != cudaSuccess)) { cudaGetLastError(); return MT_ERR_CUDA; }
+    *word = w;
+    return MT_OK;
 }
 
 int launch_attention_batch(cudaStream_t st, const void* q, const void* k_cache, const void* v_cache, void* out, const int* offsets,

@@ -214,6 +214,7 @@ bool attention_batch_supported(int hq, int hkv, int d);
 int launch_attention_batch(cudaStream_t st, const void* q, const void* k_cache, const void* v_cache, void* out, const int* offsets,
                            int batch, int m, int hq, int hkv, int d, int offset, int capacity, float scale,
                            void* workspace, size_t workspace_bytes, int dtype);
+int attention_error(unsigned* word, bool clear);
 size_t attention_workspace_bytes(int m, int hkv, int max_len);
 int launch_attention_decode(cudaStream_t st, const void* q, const void* k_cache, const void* v_cache, void* out,
                             int m, int hq, int hkv, int d, int offset, const int* offset_dev, int max_len, float scale,

@@ -164,6 +164,7 @@ def attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, off
                                          _lib.ptr(offsets), b, m, hq, hkv, d, offset, capacity, 1.0 / math.sqrt(d), _lib.ptr(ws), need,
                                          _lib.dtype_code(q.dtype))
     _lib.check(rc, "mt_attention_batch")
+    _lib.attention_devices.add(dev.index)
     return out
 
 
