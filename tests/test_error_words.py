@@ -29,7 +29,7 @@ def fake(lib_built, monkeypatch):
             state[current[-1]] = 0
         return 0
 
-    monkeypatch.setattr(_lib, "lib", types.SimpleNamespace(mt_attention_error=call))
+    monkeypatch.setattr(_lib, "lib", types.SimpleNamespace(mt_attention_error=call, mt_strerror=_lib.lib.mt_strerror))
     monkeypatch.setattr(_lib, "_workspaces", {})
     monkeypatch.setattr(_lib, "attention_devices", {0, 1})
     monkeypatch.setattr(_lib.torch.cuda, "device", Device)
