@@ -266,8 +266,9 @@ int mt_qgemm_rope_append(void* stream, const void* x, const uint32_t* qweight, c
  *   q[batch, m, hq, d] (rotated), k_cache / v_cache[batch, capacity, hkv, d] holding positions 0 .. offset_b + m - 1 of every
  *   sequence, out[batch, m, hq * d]; query i of sequence b sits at position offset_b + i and sees keys 0 .. offset_b + i.
  *   offsets_dev (device int32 [batch], may be NULL) gives every sequence its own offset_b, else `offset` holds for all.
- *   fp32 throughout, one rounding (the tensor-core kernels, d == 64 or 128, multiply the probabilities as the sum of two
- *   16-bit terms).  mt_rope_append (any even d) fills the cache of one sequence at a time.
+ *   fp32 throughout, one rounding (the tensor-core kernels, d == 64 or 128, multiply each probability as a sum of 16-bit
+ *   terms: bf16 exactly, fp16 to 2^-23 of itself or 2^-40 of the row's largest).
+ *   mt_rope_append (any even d) fills the cache of one sequence at a time.
  * mt_attention_batch: the same with a workspace of at least mt_attention_batch_workspace_bytes(m, hq, hkv, d) (0: the request
  *   uses none): up to 16 query rows per kv head (m * hq / hkv) then run on a kernel that streams the caches once, split
  *   evenly over the GPU whatever the lengths.  The workspace belongs to the call until it has run and may hold anything

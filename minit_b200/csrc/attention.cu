@@ -10,15 +10,20 @@
 //    so the key tiles of all (sequence, kv head) pairs form one line that is cut into equal runs, one per SM: sequences of
 //    different lengths keep every SM busy to the end.  mma.sync with the KEYS as the 16 rows and the query rows as the 8
 //    columns: no tensor work is spent on padding a few query rows to 16.  32 sequences of 512 to 2048 positions, 32 query and
-//    8 kv heads of 128, one token each: 45 us for 172 MB (3.8 TB/s; attention_rows_kernel 1880 us).
-//  * attention_tile_kernel, more rows: tcgen05 tiles of 128 query rows x 128 keys, accumulators and probabilities in
-//    tensor memory.  One sequence of 2000 new tokens, 32 / 8 heads of 128, bf16: 71 us (attention_rows_kernel 3360 us);
-//    4096 tokens, 64 / 8 heads: 445 us = 618 TFLOP/s of causal flops (25.8 ms).  The line between the two lies at 16 rows:
+//    8 kv heads of 128, one token each: 45.5 us for 172 MB (3.8 TB/s; attention_rows_kernel 1880 us).
+//  * attention_tile_kernel, more rows: tcgen05 tiles of 128 query rows x 64 keys (heads of 64: 128 keys), scores and
+//    probabilities in tensor memory.  One sequence of 2000 new tokens, 32 / 8 heads of 128: fp16 92 us, bf16 108 us
+//    (attention_rows_kernel 3360 us); 4096 tokens, 64 / 8 heads: fp16 612 us = 449 TFLOP/s of causal flops, bf16 745 us (25.8 ms).
+//    Two terms of both types and sums kept in tensor memory took 71 and 445 us.  The line between the two lies at 16 rows:
 //    with 32 and more the mma.sync pipe (an eighth of the tcgen05 rate) is slower than HBM.
 //
-// Scores, softmax and sums are fp32.  The tensor cores take 16-bit probabilities, so each is split into two 16-bit terms
-// (p = hi + lo, |lo| <= ulp(hi) / 2) and both are multiplied with V: the weighted sum keeps the precision of fp32
-// probabilities (2^-17 of p for bf16, 2^-22 for fp16) at the price of one more MMA.
+// Scores, softmax and sums are fp32.  The tensor cores take 16-bit probabilities, so each is split into 16-bit terms that are all
+// multiplied with V (split_terms): three of bf16, which hold an fp32 value exactly, or two of fp16, which hold it to one unit
+// of its last place (2^-23 of p), and to 2^-40 of the row's largest.  The tensor cores round their running sums towards zero: a
+// sum over thousands of keys would drift (8000 keys of one sign: 2.7e-5), so at most 128 keys are summed there and these sums are
+// added in fp32.  What is left of sums that cancel, relative to
+// sum p |v| (rms over cases of 9 to 417 keys): bf16 8e-9 to 1.6e-7, fp16 2e-8 to 1.4e-7; attention_rows_kernel 2e-8 to 3e-7 and
+// 3e-8 to 3e-7; with two bf16 terms 1.4e-7 to 9e-7.
 #include "tma.cuh"
 #include "tcgen05.cuh"
 
@@ -40,18 +45,38 @@ __device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("ba
 __device__ __forceinline__ uint32_t movmatrix(uint32_t a) {
     uint32_t d; asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a)); return d; }
 
-// two probabilities -> packed hi terms and packed lo terms
+// Two probabilities -> the packed 16-bit terms of both, largest first.  fp16 takes them times 2^15 (the sums are scaled
+// back by kUnscale): below 2^-14 an fp16 value loses bits, below 2^-25 it is zero, and a long tail of small probabilities would
+// go with it.
+constexpr float kScale = 32768.f;       // probabilities are at most 1
+template <typename T> constexpr float kUnscale = F16x2<T>::kIsBf16 ? 1.f : 1.f / kScale;
+template <typename T> constexpr int kTerms = F16x2<T>::kIsBf16 ? 3 : 2;
 template <typename T>
-__device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo) {
+__device__ __forceinline__ void split_terms(float a, float b, uint32_t (&t)[kTerms<T>]) {
     using H = F16x2<T>;
-    hi = H::pack(a, b);
-    if constexpr (H::kIsBf16) lo = H::pack(a - __uint_as_float(hi << 16), b - __uint_as_float(hi & 0xffff0000u));
-    else lo = H::pack(a - H::to_float(uint16_t(hi & 0xffff)), b - H::to_float(uint16_t(hi >> 16)));
+    if constexpr (H::kIsBf16) {                                     // cut after 8 bits, twice: 8 are left at most, and all terms are exact
+        t[0] = prmt(__float_as_uint(a), __float_as_uint(b), 0x7632u);
+        a -= __uint_as_float(__float_as_uint(a) & 0xffff0000u); b -= __uint_as_float(__float_as_uint(b) & 0xffff0000u);
+        t[1] = prmt(__float_as_uint(a), __float_as_uint(b), 0x7632u);
+        a -= __uint_as_float(__float_as_uint(a) & 0xffff0000u); b -= __uint_as_float(__float_as_uint(b) & 0xffff0000u);
+        t[2] = prmt(__float_as_uint(a), __float_as_uint(b), 0x7632u);
+    } else {
+        a *= kScale; b *= kScale;
+        t[0] = H::pack(a, b);
+        t[1] = H::pack(a - H::to_float(uint16_t(t[0] & 0xffff)), b - H::to_float(uint16_t(t[0] >> 16)));
+    }
 }
 
 // Set to 8 by a kernel of this file whose wait ran out, read by mt_attention_error.  One word per device, in the module itself: calls
 // without a workspace and calls whose scratch is gone by the time the host looks report here too.
 __device__ unsigned g_attention_error;
+
+// 32 lanes x 16 columns of tensor memory
+__device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+                   "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
 
 // On a wait that ran out: give the copies in flight time to land before the shared memory is given up.
 __device__ __forceinline__ void drain_copies() { for (int i = 0; i < 1000; ++i) __nanosleep(1000); }
@@ -262,7 +287,7 @@ attention_stream_kernel(const __grid_constant__ CUtensorMap mk, const __grid_con
                 __syncwarp();
                 if (lane == 0) mbar_arrive(kempty + 8 * st);
                 const int key0 = t * AS_KEYS + 16 * wq + g;         // keys of this lane: key0 (registers 0, 1) and key0 + 8 (2, 3)
-                uint32_t hi[NT][2], lo[NT][2];
+                uint32_t pt[NT][2][kTerms<T>];                      // B fragments of the probabilities
                 if (t * AS_KEYS + AS_KEYS > off + 1) {              // a tile that some row does not see whole
 #pragma unroll
                     for (int nt = 0; nt < NT; ++nt)
@@ -304,9 +329,9 @@ attention_stream_kernel(const __grid_constant__ CUtensorMap mk, const __grid_con
                     }
 #pragma unroll
                     for (int k2 = 0; k2 < 2; ++k2) {
-                        uint32_t ph2, pl2;
-                        split2<T>(pr[2 * k2], pr[2 * k2 + 1], ph2, pl2);
-                        hi[nt][k2] = movmatrix(ph2); lo[nt][k2] = movmatrix(pl2);      // (key, row) tile -> B fragment
+                        split_terms<T>(pr[2 * k2], pr[2 * k2 + 1], pt[nt][k2]);
+#pragma unroll
+                        for (int x = 0; x < kTerms<T>; ++x) pt[nt][k2][x] = movmatrix(pt[nt][k2][x]);      // (key, row) tile -> B fragment
                     }
                 }
                 if (!mbar_wait(vfull + 8 * st, ph, abort_flag)) { ok = false; break; }
@@ -331,8 +356,11 @@ attention_stream_kernel(const __grid_constant__ CUtensorMap mk, const __grid_con
                                  : "r"(va + (chunk >> 3) * (AS_KEYS * 128) + vrow * 128 + (((chunk & 7) ^ (vrow & 7)) << 4)));
 #pragma unroll
                     for (int nt = 0; nt < NT; ++nt) {
-                        mma16816<T>(oc[nt][j], a0, a1, a2, a3, hi[nt][0], hi[nt][1]);
-                        mma16816<T>(oc[nt][j], a0, a1, a2, a3, lo[nt][0], lo[nt][1]);
+                        float add[4] = {0.f, 0.f, 0.f, 0.f};        // small terms first, the running sum in fp32 outside the tensor core
+#pragma unroll
+                        for (int x = kTerms<T> - 1; x >= 0; --x) mma16816<T>(add, a0, a1, a2, a3, pt[nt][0][x], pt[nt][1][x]);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) oc[nt][j][e] += add[e];
                     }
                 }
                 __syncwarp();
@@ -351,7 +379,7 @@ attention_stream_kernel(const __grid_constant__ CUtensorMap mk, const __grid_con
                     float* row = merge + ((size_t)warp * C::ROWS + 8 * nt + 2 * tq + e) * C::PITCH;
                     if (g == 0) { row[D] = mx[nt][e]; row[D + 1] = v; }
 #pragma unroll
-                    for (int j = 0; j < D / 16; ++j) { row[16 * j + g] = oc[nt][j][e]; row[16 * j + 8 + g] = oc[nt][j][2 + e]; }
+                    for (int j = 0; j < D / 16; ++j) { row[16 * j + g] = oc[nt][j][e] * kUnscale<T>; row[16 * j + 8 + g] = oc[nt][j][2 + e] * kUnscale<T>; }
                 }
             bar_sync(1, AS_WARPS * 32);
             const bool whole = n == tiles;
@@ -439,11 +467,19 @@ struct TileParams {
     float c;                    // scale * log2(e)
 };
 
-template <int D> struct TileCfg {
-    static constexpr int TB = 128 * D * 2;                          // one 128-row tile of Q, K, V or the output
-    static constexpr int STAGES = 2;
-    static constexpr int OFF_K = 2 * TB, OFF_V = OFF_K + STAGES * TB;
-    static constexpr int SMEM = OFF_V + STAGES * TB + 1024;
+template <typename T, int D> struct TileCfg {
+    // Tensor memory: 512 columns hold the scores and the sums of two tiles.  The probabilities lie over the scores, 16 columns per
+    // term and 32 keys: three terms of 128 keys (192 columns) fit beside the sums of a 64-wide head, three of 64 keys (96) beside
+    // those of a 128-wide one.  Registers give the same sizes: a thread holds KEYS scores and D sums.
+    static constexpr int TERMS = kTerms<T>;
+    static constexpr int KEYS = D == 128 ? 64 : 128;                // keys per tile
+    static constexpr int S_COLS = 256 - D;                          // columns of a tile's scores / probabilities
+    static_assert(KEYS <= S_COLS && KEYS / 32 * 16 * TERMS <= S_COLS, "tensor memory");
+    static constexpr int QB = 128 * D * 2, KB = KEYS * D * 2;       // one tile of Q or the output; of K or V
+    static constexpr int STAGES = 256 / KEYS;
+    static constexpr int OFF_K = 2 * QB, OFF_V = OFF_K + STAGES * KB;
+    static constexpr int SMEM = OFF_V + STAGES * KB + 1024;
+    static constexpr int BARS = 4 * STAGES + 7;
 };
 
 // shared-memory descriptor of a [keys][64 d] tile as the MN-major operand (the d of V are the MMA's N): 128-byte rows,
@@ -452,26 +488,28 @@ __device__ __forceinline__ uint64_t desc_sw128_mn(uint32_t saddr, uint32_t half_
     return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)(half_bytes >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 
-// One CTA: two tiles of 128 query rows against the keys they see, 128 keys at a time.  Warp 0 loads (TMA), warp 1 issues the
+// One CTA: two tiles of 128 query rows against the keys they see, KEYS keys at a time.  Warp 0 loads (TMA), warp 1 issues the
 // MMAs, warpgroups 1 and 2 do the softmax of one tile each (a thread owns a row), so that one tile's softmax runs under
-// the other's MMAs.  Tensor memory: S0 | S1 | O0 | O1, 128 columns each; the probabilities overwrite the scores in place
-// (per 32 keys: 16 columns of hi terms, 16 of lo terms).
+// the other's MMAs.  Tensor memory: S0 | S1 | O0 | O1; the probabilities overwrite the scores in place (per 32 keys: 16 columns
+// of each term, largest first).  O is the sum over one tile of keys; the threads add it to the row's sums in registers when they
+// have the next tile's scores (the MMAs complete in order), so that a new maximum rescales registers only.
 template <typename T, int D>
 __global__ void __launch_bounds__(AT_THREADS, 1)
 attention_tile_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk, const __grid_constant__ CUtensorMap mv,
                       const __grid_constant__ CUtensorMap mo, const TileParams p) {
     using H = F16x2<T>;
-    using C = TileCfg<D>;
-    constexpr int TB = C::TB;
+    using C = TileCfg<T, D>;
+    constexpr int KEYS = C::KEYS, STAGES = C::STAGES, QB = C::QB, KB = C::KB, TERMS = C::TERMS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t bars[16];
+    __shared__ __align__(8) uint64_t bars[C::BARS];
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     unsigned char* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
     const uint32_t sbase = smem_u32(smem);
     const uint32_t b0 = smem_u32(bars);
-    const uint32_t qfull = b0, kfull = b0 + 8, kempty = b0 + 24, vfull = b0 + 40, vempty = b0 + 56, sfull = b0 + 72, pfull = b0 + 88, odone = b0 + 104;
+    const uint32_t qfull = b0, sfull = b0 + 8, pfull = b0 + 24, odone = b0 + 40;
+    const uint32_t kfull = b0 + 56, kempty = kfull + 8 * STAGES, vfull = kempty + 8 * STAGES, vempty = vfull + 8 * STAGES;
     volatile int* abort_flag = &s_abort;
 
     // heavy tiles first: under the causal mask the last positions have the most keys
@@ -486,7 +524,7 @@ attention_tile_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
     for (int w = 0; w < 2; ++w) {
         const int first = (2 * pair + w) * ppt, last = min(p.m, first + ppt) - 1;
         keys[w] = first < p.m ? max(1, min(off + last + 1, p.capacity)) : 0;
-        n[w] = (keys[w] + 127) / 128;
+        n[w] = (keys[w] + KEYS - 1) / KEYS;
     }
     const int nmax = max(n[0], n[1]), kmax = max(keys[0], keys[1]);
 
@@ -494,10 +532,8 @@ attention_tile_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
     if (tid == 0) {
         s_abort = 0;
         mbar_init(qfull, 1);
-        for (int i = 0; i < 2; ++i) {
-            mbar_init(kfull + 8 * i, 1); mbar_init(kempty + 8 * i, 1); mbar_init(vfull + 8 * i, 1); mbar_init(vempty + 8 * i, 1);
-            mbar_init(sfull + 8 * i, 1); mbar_init(pfull + 8 * i, 128); mbar_init(odone + 8 * i, 1);
-        }
+        for (int i = 0; i < STAGES; ++i) { mbar_init(kfull + 8 * i, 1); mbar_init(kempty + 8 * i, 1); mbar_init(vfull + 8 * i, 1); mbar_init(vempty + 8 * i, 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(sfull + 8 * i, 1); mbar_init(pfull + 8 * i, 128); mbar_init(odone + 8 * i, 1); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     tc_fence_before();
@@ -509,29 +545,29 @@ attention_tile_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
         asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
         if (warp == 0) {
             if (lane == 0) {
-                mbar_expect_tx(qfull, (n[1] > 0 ? 2 : 1) * TB);
+                mbar_expect_tx(qfull, (n[1] > 0 ? 2 : 1) * QB);
                 tma_load_5d(sbase, &mq, 0, hg * p.pack, 2 * pair * ppt, 0, b, qfull);
-                if (n[1] > 0) tma_load_5d(sbase + TB, &mq, 0, hg * p.pack, (2 * pair + 1) * ppt, 0, b, qfull);
+                if (n[1] > 0) tma_load_5d(sbase + QB, &mq, 0, hg * p.pack, (2 * pair + 1) * ppt, 0, b, qfull);
                 bool ok = true;
                 for (int j = 0; j < nmax && ok; ++j) {
-                    const int st = j & 1; const uint32_t ph = ((j >> 1) & 1) ^ 1;
+                    const int st = j % STAGES; const uint32_t ph = ((j / STAGES) & 1) ^ 1;
                     ok = mbar_wait_sleep<32>(kempty + 8 * st, ph, abort_flag);
-                    if (ok) { mbar_expect_tx(kfull + 8 * st, TB); tma_load_5d(sbase + C::OFF_K + st * TB, &mk, 0, j * 128, 0, kvh, b, kfull + 8 * st); }
+                    if (ok) { mbar_expect_tx(kfull + 8 * st, KB); tma_load_5d(sbase + C::OFF_K + st * KB, &mk, 0, j * KEYS, 0, kvh, b, kfull + 8 * st); }
                     if (ok) ok = mbar_wait_sleep<32>(vempty + 8 * st, ph, abort_flag);
-                    if (ok) { mbar_expect_tx(vfull + 8 * st, TB); tma_load_5d(sbase + C::OFF_V + st * TB, &mv, 0, j * 128, 0, kvh, b, vfull + 8 * st); }
+                    if (ok) { mbar_expect_tx(vfull + 8 * st, KB); tma_load_5d(sbase + C::OFF_V + st * KB, &mv, 0, j * KEYS, 0, kvh, b, vfull + 8 * st); }
                 }
                 if (!ok) drain_copies();
             }
             __syncwarp();
         } else if (warp == 1) {
-            const uint32_t id_qk = tc_idesc_f16(H::kIsBf16, 128, 128);
+            const uint32_t id_qk = tc_idesc_f16(H::kIsBf16, 128, KEYS);
             const uint32_t id_pv = tc_idesc_f16(H::kIsBf16, 128, D) | (1u << 16);       // B (V) MN-major
             auto qk = [&](int w, int j) {                            // S_w = Q_w K_j^T, announced on sfull[w]
                 if (lane == 0) {
 #pragma unroll
                     for (int ks = 0; ks < D / 16; ++ks) {
-                        const uint32_t o = (ks >> 2) * (128 * 128) + (ks & 3) * 32;
-                        tc_mma_ss(tmem + 128 * w, tc_desc_sw128(sbase + w * TB + o), tc_desc_sw128(sbase + C::OFF_K + (j & 1) * TB + o), id_qk, ks > 0);
+                        const uint32_t qo = (ks >> 2) * (128 * 128) + (ks & 3) * 32, ko = (ks >> 2) * (KEYS * 128) + (ks & 3) * 32;
+                        tc_mma_ss(tmem + C::S_COLS * w, tc_desc_sw128(sbase + w * QB + qo), tc_desc_sw128(sbase + C::OFF_K + (j % STAGES) * KB + ko), id_qk, ks > 0);
                     }
                     tc_commit(sfull + 8 * w);
                 }
@@ -546,15 +582,15 @@ attention_tile_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
                 __syncwarp();
             }
             for (int j = 0; j < nmax && ok; ++j) {
-                const int st = j & 1; const uint32_t ph = (j >> 1) & 1;
-                ok = mbar_wait(vfull + 8 * st, ph, abort_flag);
+                const int st = j % STAGES, sn = (j + 1) % STAGES;
+                ok = mbar_wait(vfull + 8 * st, (j / STAGES) & 1, abort_flag);
                 if (!ok) break;
-                if (j == nmax - 1 && kmax < nmax * 128) {
+                if (j == nmax - 1 && kmax < nmax * KEYS) {
                     // value rows behind the last key may hold anything (a NaN times a zero probability is a NaN): clear them
-                    for (int key = kmax - j * 128; key < 128; ++key)
+                    for (int key = kmax - j * KEYS; key < KEYS; ++key)
                         if (lane < D / 8)
                             asm volatile("st.shared.v4.b32 [%0], {%1,%1,%1,%1};"
-                                         ::"r"(sbase + C::OFF_V + st * TB + (lane >> 3) * (128 * 128) + key * 128 + ((lane & 7) << 4)), "r"(0u) : "memory");
+                                         ::"r"(sbase + C::OFF_V + st * KB + (lane >> 3) * (KEYS * 128) + key * 128 + ((lane & 7) << 4)), "r"(0u) : "memory");
                     fence_proxy_async();
                     __syncwarp();
                 }
@@ -567,17 +603,16 @@ attention_tile_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
                     tc_fence_after();
                     if (lane == 0) {
 #pragma unroll
-                        for (int ks = 0; ks < 8; ++ks) {
-                            const uint64_t vd = desc_sw128_mn(sbase + C::OFF_V + st * TB + ks * 2048, 128 * 128);
-                            const uint32_t a = tmem + 128 * w + (ks >> 1) * 32 + (ks & 1) * 8;
-                            tc_mma_ts(tmem + 256 + 128 * w, a, vd, id_pv, j > 0 || ks > 0);
-                            tc_mma_ts(tmem + 256 + 128 * w, a + 16, vd, id_pv, 1);
-                        }
+                        for (int x = TERMS - 1; x >= 0; --x)         // the small terms first: their sums lose nothing
+#pragma unroll
+                            for (int ks = 0; ks < KEYS / 16; ++ks)
+                                tc_mma_ts(tmem + 2 * C::S_COLS + D * w, tmem + C::S_COLS * w + (ks >> 1) * (16 * TERMS) + (ks & 1) * 8 + 16 * x,
+                                          desc_sw128_mn(sbase + C::OFF_V + st * KB + ks * 2048, KEYS * 128), id_pv, ks > 0 || x < TERMS - 1);
                         if (j + 1 >= n[w]) tc_commit(odone + 8 * w);
                     }
                     __syncwarp();
                     if (j + 1 < n[w]) {
-                        if (!knext) { ok = mbar_wait(kfull + 8 * (st ^ 1), ((j + 1) >> 1) & 1, abort_flag); knext = true; }
+                        if (!knext) { ok = mbar_wait(kfull + 8 * sn, ((j + 1) / STAGES) & 1, abort_flag); knext = true; }
                         if (!ok) break;
                         qk(w, j + 1);
                     }
@@ -585,7 +620,7 @@ attention_tile_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
                 if (!ok) break;
                 if (lane == 0) {
                     tc_commit(vempty + 8 * st);
-                    if (knext) tc_commit(kempty + 8 * (st ^ 1));
+                    if (knext) tc_commit(kempty + 8 * sn);
                 }
                 __syncwarp();
             }
@@ -595,66 +630,72 @@ attention_tile_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
         const int w = (warp >> 2) - 1, row = tid & 127;
         if (n[w] > 0) {
             const uint32_t lane_base = (uint32_t)(warp & 3) << 21;  // 32 TMEM lanes per warp
-            const uint32_t tS = tmem + 128 * w + lane_base, tO = tmem + 256 + 128 * w + lane_base;
+            const uint32_t tS = tmem + C::S_COLS * w + lane_base, tO = tmem + 2 * C::S_COLS + D * w + lane_base;
             const int pos = min(p.m - 1, (2 * pair + w) * ppt + row / p.pack);
             const int lim = min(off + pos + 1, p.capacity);         // keys that this row sees
             const int first_lim = off + (2 * pair + w) * ppt + 1;   // ... and that every row of the tile sees
-            float mrow = -INFINITY, l0 = 0.f, l1 = 0.f;
+            float mrow = -INFINITY, l = 0.f;
+            float acc[D], f = 0.f;                                  // sums of the tiles before the last; what to scale them by when it is added
+#pragma unroll
+            for (int e = 0; e < D; ++e) acc[e] = 0.f;
+            auto add_tile = [&]() {
+#pragma unroll
+                for (int q = 0; q < D / 32; ++q) {
+                    uint32_t o[32];
+                    tc_ld32(tO + 32 * q, o);
+                    tc_wait_ld();
+#pragma unroll
+                    for (int e = 0; e < 32; ++e) acc[32 * q + e] = fmaf(acc[32 * q + e], f, __uint_as_float(o[e]));
+                }
+            };
             bool ok = true;
             for (int j = 0; j < n[w]; ++j) {
                 ok = mbar_wait(sfull + 8 * w, j & 1, abort_flag);   // also says that P V of the tile before is complete
                 if (!ok) break;
                 tc_fence_after();
-                uint32_t s[4][32];
+                constexpr int Q = KEYS / 32;
+                uint32_t s[Q][32];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) tc_ld32(tS + 32 * q, s[q]);
+                for (int q = 0; q < Q; ++q) tc_ld32(tS + 32 * q, s[q]);
                 tc_wait_ld();
-                if (j * 128 + 128 > first_lim || j * 128 + 128 > p.capacity) {
-                    const int left = lim - j * 128;
+                if (j * KEYS + KEYS > first_lim || j * KEYS + KEYS > p.capacity) {
+                    const int left = lim - j * KEYS;
 #pragma unroll
-                    for (int q = 0; q < 4; ++q)
+                    for (int q = 0; q < Q; ++q)
 #pragma unroll
                         for (int e = 0; e < 32; ++e) if (32 * q + e >= left) s[q][e] = __float_as_uint(-INFINITY);
                 }
                 float x0 = -INFINITY, x1 = -INFINITY, x2 = -INFINITY, x3 = -INFINITY;
 #pragma unroll
-                for (int q = 0; q < 4; ++q)
+                for (int q = 0; q < Q; ++q)
 #pragma unroll
                     for (int e = 0; e < 32; e += 4) {
                         x0 = fmaxf(x0, __uint_as_float(s[q][e])); x1 = fmaxf(x1, __uint_as_float(s[q][e + 1]));
                         x2 = fmaxf(x2, __uint_as_float(s[q][e + 2])); x3 = fmaxf(x3, __uint_as_float(s[q][e + 3]));
                     }
-                const float mx = fmaxf(fmaxf(x0, x1), fmaxf(x2, x3));
-                if (j == 0) mrow = mx;
-                else if (__any_sync(0xffffffffu, (mx - mrow) * p.c > 8.f)) {
-                    // The sums are rescaled only when a row's maximum has grown by more than 8 powers of two: until then
-                    // the probabilities are taken against the old one (below 2^8, exact in the split form), and the
-                    // division by their sum at the end is against the same one.
-                    const float mn = fmaxf(mrow, mx);
-                    const float f = mrow == -INFINITY ? 0.f : ex2((mrow - mn) * p.c);
-                    mrow = mn; l0 *= f; l1 *= f;
-#pragma unroll
-                    for (int q = 0; q < D / 32; ++q) {
-                        uint32_t o[32];
-                        tc_ld32(tO + 32 * q, o);
-                        tc_wait_ld();
-#pragma unroll
-                        for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * f);
-                        tc_st32(tO + 32 * q, o);
-                    }
-                }
+                const float mn = fmaxf(mrow, fmaxf(fmaxf(x0, x1), fmaxf(x2, x3)));
+                const float fn = mrow == -INFINITY ? 0.f : ex2((mrow - mn) * p.c);
+                mrow = mn;
+                float l0 = 0.f, l1 = 0.f;                           // the tile's own sum: added key by key to a long one, small terms are lost
                 const float base = mrow == -INFINITY ? 0.f : mrow * p.c;
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    uint32_t r[32];
+                for (int q = 0; q < Q; ++q) {
+                    uint32_t r[TERMS][16];
 #pragma unroll
                     for (int e = 0; e < 16; ++e) {
                         const float a = ex2(fmaf(__uint_as_float(s[q][2 * e]), p.c, -base)), d = ex2(fmaf(__uint_as_float(s[q][2 * e + 1]), p.c, -base));
                         l0 += a; l1 += d;
-                        split2<T>(a, d, r[e], r[16 + e]);
+                        uint32_t t[TERMS];
+                        split_terms<T>(a, d, t);
+#pragma unroll
+                        for (int x = 0; x < TERMS; ++x) r[x][e] = t[x];
                     }
-                    tc_st32(tS + 32 * q, r);
+#pragma unroll
+                    for (int x = 0; x < TERMS; ++x) tc_st16(tS + 16 * (TERMS * q + x), r[x]);
                 }
+                l = fmaf(l, fn, l0 + l1);
+                if (j > 0) add_tile();
+                f = fn;
                 tc_wait_st();
                 tc_fence_before();
                 mbar_arrive(pfull + 8 * w);
@@ -662,29 +703,22 @@ attention_tile_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
             if (ok) ok = mbar_wait(odone + 8 * w, 0, abort_flag);
             if (ok) {
                 tc_fence_after();
-                const float inv = 1.f / (l0 + l1);
-                const uint32_t so = sbase + w * TB + row * 128;     // the tile's Q is no longer needed
+                add_tile();
+                const float inv = kUnscale<T> / l;
+                const uint32_t so = sbase + w * QB + row * 128;     // the tile's Q is no longer needed
 #pragma unroll
-                for (int q = 0; q < D / 32; ++q) {
-                    uint32_t o[32];
-                    tc_ld32(tO + 32 * q, o);
-                    tc_wait_ld();
+                for (int c = 0; c < D / 8; ++c) {
+                    uint32_t v[4];
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        uint32_t v[4];
-#pragma unroll
-                        for (int e = 0; e < 4; ++e)
-                            v[e] = H::pack(__uint_as_float(o[8 * c + 2 * e]) * inv, __uint_as_float(o[8 * c + 2 * e + 1]) * inv);
-                        const int chunk = (q & 1) * 4 + c;
-                        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};"
-                                     ::"r"(so + (q >> 1) * (128 * 128) + ((chunk ^ (row & 7)) << 4)), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
-                    }
+                    for (int e = 0; e < 4; ++e) v[e] = H::pack(acc[8 * c + 2 * e] * inv, acc[8 * c + 2 * e + 1] * inv);
+                    asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};"
+                                 ::"r"(so + (c >> 3) * (128 * 128) + (((c & 7) ^ (row & 7)) << 4)), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
                 }
                 fence_proxy_async();
             }
             bar_sync(1 + w, 128);
             if (row == 0 && ok && !*abort_flag) {
-                tma_store_5d(&mo, sbase + w * TB, 0, hg * p.pack, (2 * pair + w) * ppt, 0, b);          // rows past the last token are clipped
+                tma_store_5d(&mo, sbase + w * QB, 0, hg * p.pack, (2 * pair + w) * ppt, 0, b);          // rows past the last token are clipped
                 asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                 asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
             }
@@ -752,8 +786,8 @@ template <typename T, int D>
 int launch_tile_inst(cudaStream_t st, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo, const TileParams& p, unsigned grid) {
     static bool done[64] = {};
     auto kern = attention_tile_kernel<T, D>;
-    if (!set_smem(kern, TileCfg<D>::SMEM, done)) return MT_ERR_CUDA;
-    kern<<<grid, AT_THREADS, TileCfg<D>::SMEM, st>>>(mq, mk, mv, mo, p);
+    if (!set_smem(kern, TileCfg<T, D>::SMEM, done)) return MT_ERR_CUDA;
+    kern<<<grid, AT_THREADS, TileCfg<T, D>::SMEM, st>>>(mq, mk, mv, mo, p);
     return cudaGetLastError() == cudaSuccess ? MT_OK : MT_ERR_CUDA;
 }
 
@@ -812,7 +846,8 @@ int launch_attention_batch(cudaStream_t st, const void* q, const void* k_cache, 
     const long long grid = (long long)p.pairs * p.head_groups * batch;
     if (grid > 0x7fffffffLL) return MT_ERR_TOO_LARGE;
     CUtensorMap mq, mo;
-    if (!encode_rows(&mk, k_cache, dtype, d, hkv, capacity, batch, 1, 128, false) || !encode_rows(&mv, v_cache, dtype, d, hkv, capacity, batch, 1, 128, false) ||
+    const int keys = d == 128 ? TileCfg<__half, 128>::KEYS : TileCfg<__half, 64>::KEYS;      // the same for bf16
+    if (!encode_rows(&mk, k_cache, dtype, d, hkv, capacity, batch, 1, keys, false) || !encode_rows(&mv, v_cache, dtype, d, hkv, capacity, batch, 1, keys, false) ||
         !encode_rows(&mq, q, dtype, d, hq, m, batch, p.pack, ppt, true) || !encode_rows(&mo, out, dtype, d, hq, m, batch, p.pack, ppt, true)) return MT_ERR_CUDA;
     if (dtype == MT_F16)
         return d == 128 ? launch_tile_inst<__half, 128>(st, mq, mk, mv, mo, p, (unsigned)grid) : launch_tile_inst<__half, 64>(st, mq, mk, mv, mo, p, (unsigned)grid);

@@ -106,3 +106,85 @@ def test_scratch_may_hold_anything(D, d, m, hq, hkv):
         rc = _lib.lib.mt_attention_batch(_lib.current_stream(q.device), q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), offs.data_ptr(),
                                          3, m, hq, hkv, d, 0, k.shape[1], 1.0 / math.sqrt(d), ws.data_ptr(), need, 0)
         assert rc == 0 and torch.equal(out, ref)
+
+
+# ---- precision: probabilities and sums are fp32 -------------------------------------------------------------------------
+def half_ulp(v, dtype):
+    bits = 10 if dtype == torch.float16 else 7
+    return torch.exp2(torch.floor(torch.log2(v.abs().clamp_min(2.0 ** -14 if dtype == torch.float16 else 2.0 ** -126))) - bits - 1)
+
+
+@pytest.mark.parametrize("m", [1, 17])
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("dtype,gap", [(torch.float16, 22.3), (torch.float16, 24.3), (torch.bfloat16, 24.3), (torch.bfloat16, 60.0)])
+def test_long_tails_of_small_probabilities(D, m, d, dtype, gap):
+    """One key takes nearly all of the probability and has no value; tens of thousands of keys `gap` powers of two below it make
+    the result.  Their probabilities keep 2^-13 of themselves (fp16: 2^-40 / 2^-24.3 at most, 65 000 equal errors add up), and the
+    divisor the sums of whole tiles: beside half an ulp 2^-12 of the result is left."""
+    n = 65536 - m if gap < 30 else 9000
+    q = torch.zeros((1, m, 2, d), device=DEV); k = torch.zeros((1, n + m, 2, d), device=DEV)
+    q[..., 0] = 16.0
+    k[:, 3, :, 0] = gap * math.log(2.0) * math.sqrt(d) / 16.0
+    v = torch.full((1, n + m, 2, d), 1.0 if gap < 30 else 3e12, device=DEV)
+    v[:, 3] = 0.0
+    q, k, v = (t.to(dtype) for t in (q, k, v))
+    out = D.attention(q, k, v, n).double()
+    s = 16.0 * k[0, 3, 0, 0].double() / math.sqrt(d)
+    for i in range(m):
+        tail = n + i
+        ref = tail * v[0, 0, 0, 0].double() / (tail + torch.exp(s))
+        assert ((out[0, i] - ref).abs() <= 1.02 * half_ulp(ref, dtype) + 2.0 ** -12 * ref).all(), (out[0, i, 0].item(), ref.item())
+
+
+@pytest.mark.parametrize("m", [1, 17])
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_sums_that_cancel_keep_fp32_probabilities(D, dtype, d, m):
+    """Values chosen so that the weighted sum nearly vanishes: what is left is the error of the probabilities and the sums.  fp32
+    evaluation: exp2 and the scores within 2^-22 of p each, so an rms below 2^-21 of sum p |v| (two terms of bf16 alone: 2^-20.3)."""
+    b, h, n = 32, 8, 8
+    gen = torch.Generator().manual_seed(d + m)
+    total = n + m
+    q = (0.3 * torch.randn((b, m, h, d), generator=gen)).to(dtype)
+    k = torch.randn((b, total, h, d), generator=gen).to(dtype)
+    v = torch.randn((b, total, h, d), generator=gen).to(dtype).double().permute(0, 2, 1, 3).contiguous()
+    p = torch.softmax(torch.einsum("bhd,bthd->bht", q[:, -1].double(), k.double()) / math.sqrt(d), dim=-1)
+    order = p.argsort(dim=-1, descending=True)
+    for j in (0, 1, 2, total // 2):                      # each takes away what is left, to the precision of the type
+        t = order[..., j]
+        pt = p.gather(-1, t[..., None])
+        at = t[..., None, None].expand(-1, -1, 1, d)
+        rest = torch.einsum("bht,bhtd->bhd", p, v) - pt * v.gather(2, at)[:, :, 0]
+        v.scatter_(2, at, (-rest / pt).clamp(-200, 200).to(dtype).double()[:, :, None])
+    exact_sum, size = torch.einsum("bht,bhtd->bhd", p, v), torch.einsum("bht,bhtd->bhd", p, v.abs())
+    out = D.attention(q.to(DEV), k.to(DEV), v.permute(0, 2, 1, 3).contiguous().to(dtype).to(DEV), n).cpu().double().view(b, m, h, d)[:, -1]
+    err = (out - exact_sum - 0.0).pow(2).mean().sqrt() / size.pow(2).mean().sqrt()
+    assert err <= 2.0 ** -21, f"{err.item():.3g}"
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("m", [1, 17])
+def test_long_sums_do_not_drift(D, dtype, d, m):
+    """8000 values of one sign, taken back by the last key: running sums that are rounded towards zero on every step lose 2^-15 of
+    sum p |v|; sums of at most 128 keys, added in fp32, lose 2^-20 (a key tile's steps at 2^-23 each) plus 2^-21 for the scores of
+    a key whose score is 9."""
+    b, h, n = 2, 4, 8000
+    gen = torch.Generator().manual_seed(d)
+    total = n + m
+    q = torch.randn((b, m, h, d), generator=gen).to(dtype).to(DEV)
+    k = torch.randn((b, total, h, d), generator=gen).to(dtype).to(DEV)
+    v = (0.5 + torch.rand((b, total, h, d), generator=gen)).to(dtype).to(DEV)
+    q64 = q[:, -1].double()
+    scores = lambda: torch.einsum("bhd,bthd->bht", q64, k.double()) / math.sqrt(d)
+    lse = torch.logsumexp(scores()[..., :-1], dim=-1)
+    k[:, -1] = (q64 * (lse * math.sqrt(d) / q64.pow(2).sum(dim=-1))[..., None]).to(dtype)      # half of the probability
+    p = torch.softmax(scores(), dim=-1)
+    v64 = v.double()
+    for t in (total - 1, total - 2, total - 3):
+        rest = torch.einsum("bht,bthd->bhd", p, v64) - p[..., t, None] * v64[:, t]
+        v64[:, t] = (-rest / p[..., t, None]).clamp(-3000, 3000).to(dtype).double()
+    exact_sum, size = torch.einsum("bht,bthd->bhd", p, v64), torch.einsum("bht,bthd->bhd", p, v64.abs())
+    out = D.attention(q, k, v64.to(dtype), n).double().view(b, m, h, d)[:, -1]
+    err = (out - exact_sum).pow(2).mean().sqrt() / size.pow(2).mean().sqrt()
+    assert err <= 2.0 ** -20 + 2.0 ** -19, f"{err.item():.3g}"

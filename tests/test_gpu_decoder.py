@@ -214,7 +214,7 @@ def test_attention_with_one_offset_per_sequence(D):
 ])
 def test_attention_over_ragged_batches(D, dtype, m, hq, hkv, d, offs):
     """Both tensor-core kernels at the edges of their tiles and runs, against an fp64 evaluation; rows of the caches behind a
-    sequence hold NaN.  Probabilities enter as two 16-bit terms (2^-17 or better) and sums are fp32, so beside the one
+    sequence hold NaN.  Probabilities enter as 16-bit terms (2^-23 or better) and sums are fp32, so beside the one
     rounding (half an ulp) the error stays far below 2^-12 of the largest value."""
     b = len(offs)
     gen = torch.Generator().manual_seed(m * 131 + hq + d + sum(offs))
