@@ -268,7 +268,8 @@ int mt_qgemm_rope_append(void* stream, const void* x, const uint32_t* qweight, c
  *   offsets_dev (device int32 [batch], may be NULL) gives every sequence its own offset_b, else `offset` holds for all.
  *   fp32 throughout, one rounding (the tensor-core kernels, d == 64 or 128, multiply each probability as a sum of 16-bit
  *   terms: bf16 exactly, fp16 to 2^-23 of itself or 2^-40 of the row's largest).
- *   mt_rope_append (any even d) fills the cache of one sequence at a time.
+ *   Masked keys take no part, whatever they hold; an infinity or NaN that a query sees is in its result (such rows are
+ *   evaluated a second time, without tensor cores).  mt_rope_append (any even d) fills the cache of one sequence at a time.
  * mt_attention_batch: the same with a workspace of at least mt_attention_batch_workspace_bytes(m, hq, hkv, d) (0: the request
  *   uses none): up to 16 query rows per kv head (m * hq / hkv) then run on a kernel that streams the caches once, split
  *   evenly over the GPU whatever the lengths.  The workspace belongs to the call until it has run and may hold anything

@@ -10,7 +10,7 @@
 //    so the key tiles of all (sequence, kv head) pairs form one line that is cut into equal runs, one per SM: sequences of
 //    different lengths keep every SM busy to the end.  mma.sync with the KEYS as the 16 rows and the query rows as the 8
 //    columns: no tensor work is spent on padding a few query rows to 16.  32 sequences of 512 to 2048 positions, 32 query and
-//    8 kv heads of 128, one token each: 45.5 us for 172 MB (3.8 TB/s; attention_rows_kernel 1880 us).
+//    8 kv heads of 128, one token each: 46 us for 172 MB (3.8 TB/s; attention_rows_kernel 1880 us).
 //  * attention_tile_kernel, more rows: tcgen05 tiles of 128 query rows x 64 keys (heads of 64: 128 keys), scores and
 //    probabilities in tensor memory.  One sequence of 2000 new tokens, 32 / 8 heads of 128: fp16 92 us, bf16 108 us
 //    (attention_rows_kernel 3360 us); 4096 tokens, 64 / 8 heads: fp16 612 us = 449 TFLOP/s of causal flops, bf16 745 us (25.8 ms).
@@ -42,6 +42,12 @@ __device__ __forceinline__ void tma_store_5d(const CUtensorMap* map, uint32_t sr
                  ::"l"(map), "r"(src), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4) : "memory");
 }
 __device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ bool bar_or(int id, int threads, bool mine) {       // the barrier, and whether any thread said yes
+    uint32_t any;
+    asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 p, %3, 0;\nbarrier.cta.red.or.pred q, %1, %2, p;\nselp.u32 %0, 1, 0, q;\n}"
+                 : "=r"(any) : "r"(id), "r"(threads), "r"(uint32_t(mine)) : "memory");
+    return any != 0u;
+}
 __device__ __forceinline__ uint32_t movmatrix(uint32_t a) {
     uint32_t d; asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a)); return d; }
 
@@ -78,6 +84,52 @@ __device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t (&r)[16])
                    "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
 }
 
+// One output row in fp32 on the CUDA cores, by a warp (the arithmetic of attention_rows_kernel for one query): lane i returns values
+// D / 32 * i onwards.  For rows whose sums came out infinite or NaN: the tensor cores multiply every value of a key tile, so an
+// infinity or NaN that a row does not see meets its zero probabilities, and one that it sees meets zero or negative small terms.
+// Here masked keys take no part and a probability is one number: an infinity stays one, and reaches the rows that see it.
+// Out of line: sound inputs never come here, and their sums are checked once per output value.
+template <typename T, int D>
+__device__ __noinline__ void attention_row(const uint16_t* q, const uint16_t* k, const uint16_t* v, size_t pitch, int keys, float scale, float (&o)[D / 32]) {
+    using H = F16x2<T>;
+    constexpr int E = D / 32;
+    const int lane = threadIdx.x & 31;
+    float mx = -INFINITY, l = 0.f;
+#pragma unroll
+    for (int e = 0; e < E; ++e) o[e] = 0.f;
+    for (int t0 = 0; t0 < keys; t0 += 32) {
+        const int t = t0 + lane;
+        float sc = -INFINITY;
+        if (t < keys) {
+            const uint16_t* kr = k + (size_t)t * pitch;
+            sc = 0.f;
+            for (int c = 0; c < D; ++c) sc = fmaf(H::to_float(q[c]) * scale, H::to_float(kr[c]), sc);
+        }
+        float bm = sc;
+#pragma unroll
+        for (int x = 16; x > 0; x >>= 1) bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, x));
+        const float mn = fmaxf(mx, bm);
+        const float corr = mn == -INFINITY ? 1.f : __expf(mx - mn), pr = t < keys ? __expf(sc - mn) : 0.f;
+        float ps = pr;
+#pragma unroll
+        for (int x = 16; x > 0; x >>= 1) ps += __shfl_xor_sync(0xffffffffu, ps, x);
+        l = l * corr + ps;
+        mx = mn;
+#pragma unroll
+        for (int e = 0; e < E; ++e) o[e] *= corr;
+        const int cnt = min(32, keys - t0);
+        for (int j = 0; j < cnt; ++j) {
+            const float pj = __shfl_sync(0xffffffffu, pr, j);
+            const uint16_t* vr = v + (size_t)(t0 + j) * pitch + lane * E;
+#pragma unroll
+            for (int e = 0; e < E; ++e) o[e] = fmaf(pj, H::to_float(vr[e]), o[e]);
+        }
+    }
+    const float inv = 1.f / l;
+#pragma unroll
+    for (int e = 0; e < E; ++e) o[e] *= inv;
+}
+
 // On a wait that ran out: give the copies in flight time to land before the shared memory is given up.
 __device__ __forceinline__ void drain_copies() { for (int i = 0; i < 1000; ++i) __nanosleep(1000); }
 
@@ -95,12 +147,12 @@ constexpr int AS_MAX_SEGMENTS = 16384;                              // counters;
 constexpr size_t AS_PART_OFF = AS_HEAD + (size_t)AS_MAX_SEGMENTS * 4;
 
 struct StreamParams {
-    const void* q; void* out;
+    const void *q, *k, *v; void* out;
     const int* offsets;         // [batch] or null: `offset` for all
     unsigned char* ws;
     int batch, m, hq, hkv, group, offset, capacity;
     int whole;                  // 1: a (sequence, kv head) pair is never cut (no workspace counters)
-    float c;                    // scale * log2(e)
+    float scale, c;             // c: scale * log2(e)
 };
 
 template <int D, int NT> struct StreamCfg {
@@ -123,17 +175,34 @@ __device__ __forceinline__ int stream_keys(const StreamParams& p, int b) {
 __device__ __forceinline__ int stream_tiles(const StreamParams& p, int b) { return (stream_keys(p, b) + AS_KEYS - 1) / AS_KEYS; }
 
 // The stream kernel is launched programmatically behind this one and looks at the counters at the end of its first segment:
-// 32 sequences of 512 to 2048 positions 45.1 us, 46.6 behind a memset, 44.9 with counters kept between calls.
+// 32 sequences of 512 to 2048 positions 0.2 us longer than with counters kept between calls, a memset 1.7.
 __global__ void attention_zero_kernel(unsigned* counters, int n) {
     griddep_launch_dependents();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) counters[i] = 0u;
+}
+
+// all rows of pair (b, h) once more, spread over the consuming warps
+template <typename T, int D>
+__device__ __noinline__ void stream_rows(const StreamParams* p, int b, int h) {
+    const int lane = threadIdx.x & 31;
+    for (int r = threadIdx.x >> 5; r < p->m * p->group; r += AS_WARPS) {
+        const int i = r / p->group;
+        const size_t row = (((size_t)b * p->m + i) * p->hq + (size_t)h * p->group + (r - i * p->group)) * D;
+        const size_t cache = ((size_t)b * p->capacity * p->hkv + h) * D;
+        float o[D / 32];
+        attention_row<T, D>(reinterpret_cast<const uint16_t*>(p->q) + row, reinterpret_cast<const uint16_t*>(p->k) + cache,
+                            reinterpret_cast<const uint16_t*>(p->v) + cache, (size_t)p->hkv * D,
+                            min((p->offsets ? __ldg(p->offsets + b) : p->offset) + i + 1, p->capacity), p->scale, o);
+#pragma unroll
+        for (int e = 0; e < D / 32; ++e) reinterpret_cast<uint16_t*>(p->out)[row + lane * (D / 32) + e] = F16x2<T>::from_float(o[e]);
+    }
 }
 
 // Bound by HBM: one SM has to take 43 KB/us to keep up with its share, and holds six 32 KB stages in flight for that.
 // Two warps issue the copies (one K, one V: one thread alone issues about four bulk copies per microsecond).
 template <typename T, int D, int NT>
 __global__ void __launch_bounds__(AS_THREADS, 1)
-attention_stream_kernel(const __grid_constant__ CUtensorMap mk, const __grid_constant__ CUtensorMap mv, const StreamParams p) {
+attention_stream_kernel(const __grid_constant__ CUtensorMap mk, const __grid_constant__ CUtensorMap mv, const __grid_constant__ StreamParams p) {
     using H = F16x2<T>;
     using C = StreamCfg<D, NT>;
     constexpr int STAGES = C::STAGES, TB = C::TILE_BYTES;
@@ -387,10 +456,12 @@ attention_stream_kernel(const __grid_constant__ CUtensorMap mk, const __grid_con
             auto slot = [&](long long cta) {                        // a CTA's partial of this segment: 0 when its run starts in it, else 1
                 return reinterpret_cast<float*>(p.ws + AS_PART_OFF) + ((size_t)cta * 2 + (cta * per >= seg_first ? 0 : 1)) * C::ROWS * C::PITCH;
             };
+            float zero = 0.f;                                       // stays so unless a stored value is infinite or NaN
             auto store = [&](int r, int d, float l, float a) {
                 const int mi = r / p.group;
-                reinterpret_cast<uint16_t*>(p.out)[(((size_t)b * p.m + mi) * p.hq + (size_t)h * p.group + (r - mi * p.group)) * D + d] =
-                    H::from_float(a / l);
+                const float v = a / l;
+                zero = fmaf(v, 0.f, zero);
+                reinterpret_cast<uint16_t*>(p.out)[(((size_t)b * p.m + mi) * p.hq + (size_t)h * p.group + (r - mi * p.group)) * D + d] = H::from_float(v);
             };
             for (int e = tid; e < R * D; e += AS_WARPS * 32) {
                 const int r = e / D, d = e % D;
@@ -438,7 +509,7 @@ attention_stream_kernel(const __grid_constant__ CUtensorMap mk, const __grid_con
                 }
             }
             if (tid == 0) s_stop = *abort_flag;                     // one answer for all warps: they leave the loop together
-            bar_sync(1, AS_WARPS * 32);                             // the merge rows are free again
+            if (bar_or(1, AS_WARPS * 32, !(zero == 0.f))) stream_rows<T, D>(&p, b, h);      // the merge rows are free again
             ok = s_stop == 0;
             seg_first += tiles;
             t = 0;
@@ -459,12 +530,13 @@ attention_stream_kernel(const __grid_constant__ CUtensorMap mk, const __grid_con
 constexpr int AT_THREADS = 384;
 
 struct TileParams {
+    const void *q, *k, *v;
     const int* offsets;
     unsigned* err;
     int batch, m, hq, hkv, group, offset, capacity;
     int pack;                   // query heads of one kv head that share a tile: row = position * pack + head
     int head_groups, pairs;     // hq / pack; pairs of 128-row tiles per (sequence, head group)
-    float c;                    // scale * log2(e)
+    float scale, c;             // c: scale * log2(e)
 };
 
 template <typename T, int D> struct TileCfg {
@@ -650,7 +722,7 @@ attention_tile_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
             };
             bool ok = true;
             for (int j = 0; j < n[w]; ++j) {
-                ok = mbar_wait(sfull + 8 * w, j & 1, abort_flag);   // also says that P V of the tile before is complete
+                ok = __all_sync(0xffffffffu, mbar_wait(sfull + 8 * w, j & 1, abort_flag));      // also says that P V of the tile before is complete
                 if (!ok) break;
                 tc_fence_after();
                 constexpr int Q = KEYS / 32;
@@ -700,19 +772,39 @@ attention_tile_kernel(const __grid_constant__ CUtensorMap mq, const __grid_const
                 tc_fence_before();
                 mbar_arrive(pfull + 8 * w);
             }
-            if (ok) ok = mbar_wait(odone + 8 * w, 0, abort_flag);
+            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(odone + 8 * w, 0, abort_flag));
             if (ok) {
                 tc_fence_after();
                 add_tile();
                 const float inv = kUnscale<T> / l;
-                const uint32_t so = sbase + w * QB + row * 128;     // the tile's Q is no longer needed
+                const uint32_t so = sbase + w * QB;                 // the tile's Q is no longer needed
+                float zero = 0.f;                                   // stays so unless a value is infinite or NaN
 #pragma unroll
                 for (int c = 0; c < D / 8; ++c) {
                     uint32_t v[4];
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) v[e] = H::pack(acc[8 * c + 2 * e] * inv, acc[8 * c + 2 * e + 1] * inv);
+                    for (int e = 0; e < 4; ++e) {
+                        const float v0 = acc[8 * c + 2 * e] * inv, v1 = acc[8 * c + 2 * e + 1] * inv;
+                        zero = fmaf(v0, 0.f, fmaf(v1, 0.f, zero));
+                        v[e] = H::pack(v0, v1);
+                    }
                     asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};"
-                                 ::"r"(so + (c >> 3) * (128 * 128) + (((c & 7) ^ (row & 7)) << 4)), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
+                                 ::"r"(so + row * 128 + (c >> 3) * (128 * 128) + (((c & 7) ^ (row & 7)) << 4)), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
+                }
+                for (unsigned bad = __ballot_sync(0xffffffffu, !(zero == 0.f)); bad != 0u; bad &= bad - 1u) {
+                    const int r = (warp & 3) * 32 + __ffs(bad) - 1, i = (2 * pair + w) * ppt + r / p.pack;
+                    if (i >= p.m) continue;                         // behind the last token: never stored
+                    float o[D / 32];
+                    const size_t cache = ((size_t)b * p.capacity * p.hkv + kvh) * D;
+                    attention_row<T, D>(reinterpret_cast<const uint16_t*>(p.q) + (((size_t)b * p.m + i) * p.hq + hg * p.pack + r % p.pack) * D,
+                                        reinterpret_cast<const uint16_t*>(p.k) + cache, reinterpret_cast<const uint16_t*>(p.v) + cache, (size_t)p.hkv * D,
+                                        min(off + i + 1, p.capacity), p.scale, o);
+                    const int d0 = lane * (D / 32);
+                    __syncwarp();
+#pragma unroll
+                    for (int e = 0; e < D / 32; e += 2)
+                        asm volatile("st.shared.b32 [%0], %1;" ::"r"(so + r * 128 + (d0 >> 6) * (128 * 128) + ((((d0 >> 3) & 7) ^ (r & 7)) << 4) + ((d0 & 7) + e) * 2),
+                                     "r"(H::pack(o[e], o[e + 1])) : "memory");
                 }
                 fence_proxy_async();
             }
@@ -815,9 +907,13 @@ int launch_attention_batch(cudaStream_t st, const void* q, const void* k_cache, 
     const int group = hq / hkv;
     const float c = scale * 1.4426950408889634f;
     CUtensorMap mk, mv;
-    if (workspace && (long long)m * group <= 16 && workspace_bytes >= attention_batch_workspace_bytes(m, hq, hkv, d)) {
+    // rows that are evaluated a second time read q again behind the first store: with out in q's place the tile kernel, which
+    // stores a row once, takes the call
+    const size_t bytes = (size_t)batch * m * hq * d * 2;
+    const bool apart = static_cast<const char*>(q) + bytes <= static_cast<const char*>(out) || static_cast<const char*>(out) + bytes <= static_cast<const char*>(q);
+    if (workspace && apart && (long long)m * group <= 16 && workspace_bytes >= attention_batch_workspace_bytes(m, hq, hkv, d)) {
         StreamParams p;
-        p.q = q; p.out = out; p.offsets = offsets; p.ws = static_cast<unsigned char*>(workspace);
+        p.q = q; p.k = k_cache; p.v = v_cache; p.out = out; p.offsets = offsets; p.scale = scale; p.ws = static_cast<unsigned char*>(workspace);
         p.batch = batch; p.m = m; p.hq = hq; p.hkv = hkv; p.group = group; p.offset = offset; p.capacity = capacity; p.c = c;
         p.whole = (long long)batch * hkv > AS_MAX_SEGMENTS;
         if (!p.whole) {
@@ -836,6 +932,7 @@ int launch_attention_batch(cudaStream_t st, const void* q, const void* k_cache, 
 #undef MT_STREAM
     }
     TileParams p;
+    p.q = q; p.k = k_cache; p.v = v_cache; p.scale = scale;
     p.offsets = offsets; p.err = workspace_bytes >= 4 ? static_cast<unsigned*>(workspace) : nullptr;
     p.batch = batch; p.m = m; p.hq = hq; p.hkv = hkv; p.group = group; p.offset = offset; p.capacity = capacity; p.c = c;
     p.pack = 1;

@@ -188,3 +188,44 @@ def test_long_sums_do_not_drift(D, dtype, d, m):
     out = D.attention(q, k, v64.to(dtype), n).double().view(b, m, h, d)[:, -1]
     err = (out - exact_sum).pow(2).mean().sqrt() / size.pow(2).mean().sqrt()
     assert err <= 2.0 ** -20 + 2.0 ** -19, f"{err.item():.3g}"
+
+
+# ---- infinities and NaN -------------------------------------------------------------------------------------------------
+def same(out, ref, dtype):
+    """Infinities and NaN where the reference has them; elsewhere half an ulp and 2^-12 of the largest finite value."""
+    out = out.double()
+    fin = torch.isfinite(ref)
+    assert torch.equal(torch.isnan(out), torch.isnan(ref))
+    assert torch.equal(out[torch.isinf(ref)], ref[torch.isinf(ref)])
+    size = ref[fin].abs().max()
+    assert ((out - ref)[fin].abs() <= 1.02 * half_ulp(ref[fin], dtype) + 2.0 ** -12 * size).all()
+
+
+@pytest.mark.parametrize("m,hq,hkv,offs", [(2, 8, 2, [300, 63, 0]), (40, 8, 2, [100, 0]), (150, 4, 4, [7])])
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_infinities_and_nan_reach_the_rows_that_see_them(D, dtype, d, m, hq, hkv, offs):
+    """An infinite value under a positive probability is the result; a value or key that is not a number makes the rows that see it
+    so, and no other: rows before it, in the same tile of rows, are what they are without it."""
+    q, k, v, dev_offs = inputs(len(offs), m, hq, hkv, d, offs, dtype, seed=5)
+    last = offs[0] + m - 1
+    for value, where, t in ((math.inf, "v", 0), (-math.inf, "v", last), (math.nan, "v", last - m // 2), (math.nan, "k", last), (math.inf, "k", last - 1)):
+        kk, vv = k.clone(), v.clone()
+        (vv if where == "v" else kk)[0, t, 0, 5] = value
+        same(D.attention(q, kk, vv, offsets=dev_offs), exact(q, kk, vv, offs), dtype)
+    vv = v.clone()
+    vv[0, 0, 0, 5], vv[0, min(1, last), 0, 5], vv[0, 0, 0, 6] = math.inf, -math.inf, 65000.0
+    same(D.attention(q, k, vv, offsets=dev_offs), exact(q, k, vv, offs), dtype)
+    qq = q.clone()
+    qq[0, m - 1, 1, 3] = math.nan                       # one query of one head
+    same(D.attention(qq, k, v, offsets=dev_offs), exact(qq, k, v, offs), dtype)
+    torch.testing.assert_close(D.attention(q, k, v, offsets=dev_offs).double(), exact(q, k, v, offs), rtol=2e-2, atol=2e-2)
+
+
+@pytest.mark.parametrize("m", [1, 40])
+def test_result_in_the_place_of_the_queries(D, m):
+    """out may be the queries' own memory, with infinities too (such rows are evaluated a second time from q)."""
+    q, k, v, offs = inputs(2, m, 8, 2, 128, [200, 31], seed=11)
+    v[0, 3, 1, 7] = math.inf
+    buf = q.clone()
+    same(D.attention(buf, k, v, offsets=offs, out=buf.view(2, m, -1)), exact(q, k, v, [200, 31]), torch.float16)
