@@ -531,7 +531,8 @@ int mt_attention_batch(void* stream, const void* q, const void* k_cache, const v
     int rc = check_device();
     if (rc != MT_OK) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (attention_batch_supported(hq, hkv, d))
+    // the tensor-core kernels take a row's maximum before they scale: only for a scale above zero (and finite times log2(e)) is it the same
+    if (attention_batch_supported(hq, hkv, d) && scale > 0.f && scale <= 1e38f)
         return launch_attention_batch(st, q, k_cache, v_cache, out, offsets_dev, batch, m, hq, hkv, d, offset, capacity, scale,
                                       workspace, workspace_bytes, dtype);
     return launch_attention_rows(st, q, k_cache, v_cache, out, offsets_dev, batch, m, hq, hkv, d, offset, capacity, scale, dtype);

@@ -229,3 +229,19 @@ def test_result_in_the_place_of_the_queries(D, m):
     v[0, 3, 1, 7] = math.inf
     buf = q.clone()
     same(D.attention(buf, k, v, offsets=offs, out=buf.view(2, m, -1)), exact(q, k, v, [200, 31]), torch.float16)
+
+
+# ---- ends of the arguments' ranges --------------------------------------------------------------------------------------
+@pytest.mark.parametrize("m", [1, 20])
+@pytest.mark.parametrize("scale", [-0.2, 0.0, 1e-42])
+def test_any_scale(D, m, scale):
+    """The C call takes any scale: below zero the largest score is the smallest product, at zero all keys weigh the same."""
+    from minit_b200 import _lib
+    q, k, v, offs = inputs(2, m, 8, 2, 128, [150, 64], seed=21)
+    need = _lib.lib.mt_attention_batch_workspace_bytes(m, 8, 2, 128)
+    ws = torch.empty(max(need, 16), dtype=torch.uint8, device=DEV)
+    out = torch.empty((2, m, 8 * 128), dtype=torch.float16, device=DEV)
+    rc = _lib.lib.mt_attention_batch(_lib.current_stream(q.device), q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), offs.data_ptr(),
+                                     2, m, 8, 2, 128, 0, k.shape[1], scale, ws.data_ptr(), need, 0)
+    assert rc == 0
+    same(out, exact(q, k, v, [150, 64], scale), torch.float16)
