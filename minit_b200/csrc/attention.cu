@@ -357,7 +357,7 @@ attention_stream_kernel(const __grid_constant__ CUtensorMap mk, const __grid_con
                 if (lane == 0) mbar_arrive(kempty + 8 * st);
                 const int key0 = t * AS_KEYS + 16 * wq + g;         // keys of this lane: key0 (registers 0, 1) and key0 + 8 (2, 3)
                 uint32_t pt[NT][2][kTerms<T>];                      // B fragments of the probabilities
-                if (t * AS_KEYS + AS_KEYS > off + 1) {              // a tile that some row does not see whole
+                if (t * AS_KEYS + AS_KEYS > min(off + 1, keys)) {   // a tile that some row does not see whole, or that ends behind the cache
 #pragma unroll
                     for (int nt = 0; nt < NT; ++nt)
 #pragma unroll

@@ -245,3 +245,14 @@ def test_any_scale(D, m, scale):
                                      2, m, 8, 2, 128, 0, k.shape[1], scale, ws.data_ptr(), need, 0)
     assert rc == 0
     same(out, exact(q, k, v, [150, 64], scale), torch.float16)
+
+
+@pytest.mark.parametrize("m", [2, 20])
+@pytest.mark.parametrize("d", [64, 128])
+def test_offsets_past_the_capacity(D, m, d):
+    """A device offset of the capacity or more: every query sees the whole cache, and nothing behind it."""
+    q, k, v, _ = inputs(3, m, 8, 2, d, [101 - m] * 3, seed=31)
+    offs = [101, 5000, 101 - m]
+    out = D.attention(q, k - 3.0, v, offsets=torch.tensor(offs, dtype=torch.int32, device=DEV))
+    clamped = torch.cat([exact(q[s:s + 1, i:i + 1], k[s:s + 1] - 3.0, v[s:s + 1], [min(offs[s] + i, 100)]) for s in range(3) for i in range(m)], dim=1)
+    same(out.view(1, 3 * m, -1), clamped, torch.float16)
