@@ -32,30 +32,36 @@ __device__ __forceinline__ uint32_t mbar_test(uint32_t bar, uint32_t parity) {
                  : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok;
 }
-// Bounded wait: spins, then backs off with nanosleep; gives up after roughly a second.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-    for (int i = 0; i < 4096; ++i) if (mbar_try_wait(bar, parity)) return true;
-    for (int i = 0; i < (1 << 22); ++i) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if (*abort_flag) return false;
-        __nanosleep(128);
-    }
-    *abort_flag = 1;
+// Whether a wait has to be given up: another role already has, or a second has passed on the GPU's clock since the first call
+// (`since`: 0 before it).  Raises the abort flag.  Neither try_wait nor nanosleep says how long it takes, so a number of tries is
+// no bound in time.
+constexpr uint32_t kWaitNs = 1000000000u;
+__device__ __forceinline__ bool wait_over(uint32_t& since, volatile int* abort_flag) {
+    if (*abort_flag) return true;
+    uint32_t now;
+    asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(now));
+    if (since == 0u) since = now | 1u;
+    else if (now - since > kWaitNs) { *abort_flag = 1; return true; }
     return false;
 }
-// Bounded wait that SLEEPS between looks.  A warp that spins on try_wait takes issue slots from the warps of its
-// scheduler and keeps the barrier unit busy; roles that wait long by design (an epilogue waiting for a whole tile, a
-// producer that runs stages ahead) look every NS nanoseconds instead, and roles on the critical path every few tens.
+// Bounded wait: try_wait parks the thread in hardware and wakes it when the phase completes.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+    uint32_t since = 0u;
+    for (uint32_t i = 1u;; ++i) {
+        if (mbar_try_wait(bar, parity)) return true;
+        if ((i & 63u) == 0u && wait_over(since, abort_flag)) return false;
+    }
+}
+// Bounded wait that SLEEPS between looks (up to twice NS nanoseconds): for roles that wait long by design and whose wake-up is
+// on nobody's critical path.
 template <int NS>
 __device__ __forceinline__ bool mbar_wait_sleep(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-    constexpr int LIMIT = NS >= 256 ? (1 << 22) : (1 << 25);          // about a second either way
-    for (int i = 0; i < LIMIT; ++i) {
+    uint32_t since = 0u;
+    for (uint32_t i = 1u;; ++i) {
         if (mbar_test(bar, parity)) return true;
-        if ((i & 63) == 63 && *abort_flag) return false;
+        if ((i & 63u) == 0u && wait_over(since, abort_flag)) return false;
         __nanosleep(NS);
     }
-    *abort_flag = 1;
-    return false;
 }
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
