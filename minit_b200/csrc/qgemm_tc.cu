@@ -893,6 +893,10 @@ bool tc_tmem_a_preferred(int m, int n, int bits) {
     return bits == 4 && m > 64 && m <= 128 && (n + 255) / 256 >= 100;
 }
 
+// The SMs of a B200.  How a request is cut decides how much workspace it needs, so the sizes that a caller asks for, the check of
+// what it brings and the launch count with this one number, whatever device is current (a part with more or fewer SMs runs
+// the same items on a grid of its own size).
+constexpr int kPlanSms = 148;
 // Time of one wave of parts of tiles of bm rows cut into s parts along K, in k-blocks (about 0.45 us): the part's own k-blocks
 // and, when there is more than one part, its fp32 partial tile (written, handed over in groups of rows, read back): measured
 // 4 us with 64-row tiles, 11 us with 192-row tiles.
@@ -900,24 +904,23 @@ static double tcx_cost(int bm, int kblocks, int s) { return double((kblocks + s 
 // Parts per tile of the last, partly filled wave of 256-column tiles (1: leave it alone); a request of fewer tiles than SMs is
 // one such wave.  The parts stay in one wave: cut into two waves, 14336 x 4096 at 1000 rows (96 tiles) took 145 us as 288 parts
 // against 134 uncut, 4096 x 28672 at 1000 rows 239 against 206 (a second wave's start is not hidden behind the first's end).
-int tcx_tail_split(int m, int n, int k, int sms, int bm) {
+int tcx_tail_split(int m, int n, int k, int bm) {
     const int tiles = ((n + 255) / 256) * ((m + bm - 1) / bm);
-    const int rest = tiles % sms;
+    const int rest = tiles % kPlanSms;
     if (rest == 0) return 1;
     const int kblocks = (k + TC_BK - 1) / TC_BK;
     int best = 1;
-    for (int s = 2; s <= 8 && kblocks >= 8 * s && rest * s <= sms; ++s)
+    for (int s = 2; s <= 8 && kblocks >= 8 * s && rest * s <= kPlanSms; ++s)
         if (tcx_cost(bm, kblocks, s) < tcx_cost(bm, kblocks, best)) best = s;
     return best;
 }
 size_t tcx_workspace_bytes(int m, int n, int k) {
-    const int sms = 148;
     size_t need = 0;
     for (int bm : {192, 160}) {
-        const int split = tcx_tail_split(m, n, k, sms, bm);
+        const int split = tcx_tail_split(m, n, k, bm);
         if (split <= 1) continue;
         const int tiles = ((n + 255) / 256) * ((m + bm - 1) / bm);
-        const size_t b = (size_t)(tiles % sms) * split * 2 * bm * 128 * 4;
+        const size_t b = (size_t)(tiles % kPlanSms) * split * 2 * bm * 128 * 4;
         if (b > need) need = b;
     }
     return need;
@@ -925,11 +928,11 @@ size_t tcx_workspace_bytes(int m, int n, int k) {
 // Rows per tile: 192 (two A slots) or 160 (three).  Whole waves, then the last one cut along K, in row x k-block units; the
 // 160-row tile is charged 12 % (4096 rows of three shapes: 1099 / 1113 / 1099 TFLOP/s with 192 rows, 1044 / 1106 / 993 with 160;
 // 4096 x 28672 at 1000 rows 224 us and 235), and wins where it pads less (that shape at 800 rows: 184 -> 173 us).
-static int tcx_rows_per_tile(int m, int n, int k, int sms) {
+static int tcx_rows_per_tile(int m, int n, int k) {
     auto cost = [&](int bm) {
         const int tiles = ((n + 255) / 256) * ((m + bm - 1) / bm), kblocks = (k + TC_BK - 1) / TC_BK;
-        const int rest = tiles % sms, s = tcx_tail_split(m, n, k, sms, bm);
-        return bm * (bm == 160 ? 1.12 : 1.0) * (double(tiles / sms) * kblocks + (rest ? tcx_cost(bm, kblocks, s) : 0.0));
+        const int rest = tiles % kPlanSms, s = tcx_tail_split(m, n, k, bm);
+        return bm * (bm == 160 ? 1.12 : 1.0) * (double(tiles / kPlanSms) * kblocks + (rest ? tcx_cost(bm, kblocks, s) : 0.0));
     };
     return cost(160) < cost(192) ? 160 : 192;
 }
@@ -985,8 +988,8 @@ static int launch_tc_inst(cudaStream_t st, const QGemmArgs& a, const CUtensorMap
     return cudaGetLastError() == cudaSuccess ? MT_OK : MT_ERR_CUDA;
 }
 
-// Launch of qgemm_tcx_kernel with tiles of 256 columns x bm rows.  split_all == 0: one item per tile, the tiles of a last
-// wave that is at most half full cut along K (tcx_tail_split); split_all > 0: EVERY tile cut into that many parts (the
+// Launch of qgemm_tcx_kernel with tiles of 256 columns x bm rows.  split_all == 0: one item per tile, the tiles of a last,
+// partly filled wave cut along K (tcx_tail_split); split_all > 0: EVERY tile cut into that many parts (the
 // schedule for few, deep tiles).  `mq` is the packed-weight map with the 256-column box; `p` holds the common fields.
 static int launch_tcx(cudaStream_t st, const QGemmArgs& a, EncodeTiledFn enc, const CUtensorMap& mq, TcParams p, int bm, int split_all, int bk = TC_BK) {
     CUtensorMap mxb;
@@ -1020,8 +1023,8 @@ static int launch_tcx(cudaStream_t st, const QGemmArgs& a, EncodeTiledFn enc, co
         if (!ws_ok || a.workspace_bytes < kCounterBytes + need || tiles * 8 > kMaxTiles - 8) return MT_ERR_WORKSPACE;
         p.full_tiles = 0; p.split = split_all;
     } else {
-        const int split = bm > 64 ? tcx_tail_split(a.m, a.n, a.k, sms, bm) : 1;
-        const int rest = tiles % sms;
+        const int split = bm > 64 ? tcx_tail_split(a.m, a.n, a.k, bm) : 1;
+        const int rest = tiles % kPlanSms;
         const size_t need = (size_t)rest * split * 2 * bm * 128 * 4;
         if (split > 1 && ws_ok && a.workspace_bytes >= kCounterBytes + need && rest * 8 <= kMaxTiles - 8) {
             p.full_tiles = tiles - rest; p.split = split;
@@ -1055,16 +1058,16 @@ static int launch_tcx(cudaStream_t st, const QGemmArgs& a, EncodeTiledFn enc, co
 // tile is cut into `split` parts along K so that the parts fill the GPU's waves (few, deep tiles otherwise: 224 tiles of
 // 128 k-blocks on 8192 x 57344, 32 tiles of 448 on 28672 x 8192).
 static int tcx_rows_bm(int m) { return m <= 64 ? 64 : (m <= 160 ? 160 : 192); }
-static int tcx_rows_split(int m, int n, int k, int sms) {
+static int tcx_rows_split(int m, int n, int k) {
     const int tiles = (n + 255) / 256;
     const int kblocks = (k + TC_BK - 1) / TC_BK;
     int best = 1;
-    for (int s = 2; s <= 8 && kblocks >= 8 * s && tiles * s <= sms; ++s)
+    for (int s = 2; s <= 8 && kblocks >= 8 * s && tiles * s <= kPlanSms; ++s)
         if (tcx_cost(tcx_rows_bm(m), kblocks, s) < tcx_cost(tcx_rows_bm(m), kblocks, best)) best = s;
     return best;
 }
 size_t tcx_rows_workspace_bytes(int m, int n, int k) {
-    const int s = tcx_rows_split(m, n, k, 148);
+    const int s = tcx_rows_split(m, n, k);
     return s > 1 ? (size_t)((n + 255) / 256) * s * 2 * tcx_rows_bm(m) * 128 * 4 : 0;
 }
 bool tcx_rows_supported(const QGemmArgs& a) {
@@ -1096,10 +1099,7 @@ int launch_tcx_rows(cudaStream_t st, const QGemmArgs& a) {
     p.err = static_cast<unsigned*>(a.workspace) + (kMaxTiles - 1);
     p.m = a.m; p.n = a.n; p.k = a.k; p.groups = a.groups; p.gs = a.k / a.groups;
     p.zp1_const = 1 << (a.bits - 1);
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    int split = tcx_rows_split(a.m, a.n, a.k, sms);
+    int split = tcx_rows_split(a.m, a.n, a.k);
     if (((a.flags >> 16) & 0xff) != 0) split = std::min((a.flags >> 16) & 0xff, a.k / bk);      // tuning: MT_FLAG_SPLITS forces the parts per tile
     return launch_tcx(st, a, enc, mq, p, tcx_rows_bm(a.m), split, bk);
 }
@@ -1141,23 +1141,23 @@ int launch_tc(cudaStream_t st, const QGemmArgs& a) {
     p.m = a.m; p.n = a.n; p.k = a.k; p.groups = a.groups; p.gs = a.k / a.groups;
     p.n_tiles = (a.n + TC_BN - 1) / TC_BN; p.m_tiles = (a.m + bm - 1) / bm;
     p.zp1_const = 1 << (a.bits - 1);
-    // Two int4 prefill tiles: 256 x 192 with the dequantized weights in tensor memory (about 8 % faster per unit of work)
-    // and 256 x 256 with them in shared memory.  Both run one tile per CTA at a time on a persistent grid, so the one
-    // whose tile count fills the last wave better wins: compare waves x rows per tile.
-    // From 65 to 128 rows only the first has a tile that fits (the 256 x 256 one would be half empty), and it pays when
-    // its single row of tiles nearly fills the GPU (tc_tmem_a_preferred): 8192 x 57344 at 128 rows 196 us against 336 us
+    // Above 192 rows, and below where the one-row schedule did not fit (N < 256, no workspace for its parts).  Two int4 tiles:
+    // 256 x 192 / 160 with the dequantized weights in tensor memory (about 8 % faster per unit of work) and 256 x 256 with them in
+    // shared memory.  Both run one tile per CTA at a time on a persistent grid, so the one whose tile count fills the last
+    // wave better wins: compare waves x rows per tile.  Up to 128 rows, uncut, only the first has a tile that fits, and it pays
+    // when its single row of tiles nearly fills the GPU (tc_tmem_a_preferred): 8192 x 57344 at 128 rows 196 us against 336 us
     // for the mid-batch kernel, but 28672 x 8192 (32 tiles) 309 us against 218 us.
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int xbm = ((a.flags >> 28) & 1) ? 160 : tcx_rows_per_tile(a.m, a.n, a.k, sms);      // bit 28 of the flags: always 160 (tuning)
+    const int xbm = ((a.flags >> 28) & 1) ? 160 : tcx_rows_per_tile(a.m, a.n, a.k);      // bit 28 of the flags: always 160 (tuning)
     bool tmem_a = (a.flags & MT_FLAG_TC_TMEM_A) != 0 || (wide && a.m <= 128 && tc_tmem_a_preferred(a.m, a.n, a.bits)) ||
                   (wide && a.m > 128 && a.bits == 8 && !(a.flags & MT_FLAG_TC_SMEM_A));      // three 88 KB stages of the other tile do not fit for 8 bits
     if (wide && a.m > 128 && !tmem_a && !(a.flags & MT_FLAG_TC_SMEM_A)) {
-        const long long waves_w = ((long long)((a.n + 255) / 256) * ((a.m + TCW_BM - 1) / TCW_BM) + sms - 1) / sms;
-        const int kblocks = a.k / TC_BK, tiles_x = ((a.n + 255) / 256) * ((a.m + xbm - 1) / xbm), rest = tiles_x % sms;
-        const int split = tcx_tail_split(a.m, a.n, a.k, sms, xbm);
-        const double cost_x = xbm * (double(tiles_x / sms) * kblocks + (rest ? tcx_cost(xbm, kblocks, split) : 0.0));
+        const long long waves_w = ((long long)((a.n + 255) / 256) * ((a.m + TCW_BM - 1) / TCW_BM) + kPlanSms - 1) / kPlanSms;
+        const int kblocks = a.k / TC_BK, tiles_x = ((a.n + 255) / 256) * ((a.m + xbm - 1) / xbm), rest = tiles_x % kPlanSms;
+        const int split = tcx_tail_split(a.m, a.n, a.k, xbm);
+        const double cost_x = xbm * (double(tiles_x / kPlanSms) * kblocks + (rest ? tcx_cost(xbm, kblocks, split) : 0.0));
         tmem_a = cost_x * 0.92 <= double(waves_w) * TCW_BM * kblocks;
     }
     if (wide && (tmem_a || (a.m > 128 && a.bits == 4))) {   // the packed-weight box covers 256 columns

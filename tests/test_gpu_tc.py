@@ -209,3 +209,23 @@ def test_scales_of_the_right_group_every_time(M, gs, m, bits):
     d = to_dev(c, DEV)
     for _ in range(20):
         assert torch.equal(M.quantized_matrix_multiply(d["x"], d["qweight"], d["qzeros"], d["scales"], None, bits=bits), ref)
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("k,n,m", [(8192, 19 * 256, 32), (8192, 19 * 256, 150), (4096, 1024, 17), (14336, 4096, 1000), (4096, 28672, 400), (11008, 4096, 192)])
+def test_the_workspace_that_is_asked_for_is_enough(M, k, n, m, bits):
+    """A C caller that brings exactly mt_workspace_bytes gets the same bits as one that brings more: the parts per tile are counted
+    the same way where the size is asked for and where the kernel is launched."""
+    from minit_b200 import _lib
+    d = to_dev(O.make_gptq_case(k, n, m, bits=bits, seed=k + n + m), DEV)
+    outs = []
+    for extra in (0, 64 << 20):
+        ws = torch.zeros(_lib.lib.mt_workspace_bytes(m, n, k, bits) + extra, dtype=torch.uint8, device=DEV)
+        out = torch.zeros((m, n), dtype=torch.float16, device=DEV)
+        rc = _lib.lib.mt_qgemm(_lib.current_stream(out.device), d["x"].data_ptr(), d["qweight"].data_ptr(), None, d["qzeros"].data_ptr(), d["scales"].data_ptr(),
+                               None, out.data_ptr(), m, n, k, k // 128, bits, 0, ws.data_ptr(), ws.numel(), 0)
+        assert rc == 0
+        torch.cuda.synchronize()
+        assert int(ws[:_lib.COUNTER_BYTES].view(torch.int32).abs().sum().item()) == 0
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1])
