@@ -89,7 +89,7 @@ constexpr int DQ_WARPS = 4, DQ_ROWS = 8;         // packed rows per warp: 64 (32
 
 }  // namespace
 
-// grid: (256-column windows, runs of DQ_WARPS * DQ_ROWS packed rows); output rows are `pitch` values apart.  A packed row whose
+// grid: (256-column windows, runs of DQ_WARPS * DQ_ROWS packed rows over y and z); output rows are `pitch` values apart.  A packed row whose
 // values of k all belong to one group (contiguous groups, or a g_idx that is) uses one set of constants per group; a mixed
 // row (act-order) fetches the constants of every k: a block's window of scales and zeros (20 KB for 32 groups) stays in L1.
 template <int BITS, typename T>
@@ -102,7 +102,8 @@ dequant_kernel(const uint32_t* __restrict__ qweight, const int32_t* __restrict__
     const bool live = (blockIdx.x * 32 + lane) * 8 < n;           // lanes past the last column stay for the warp's shuffles
     const int c = live ? (blockIdx.x * 32 + lane) * 8 : 0;
     const int kp = k / PACK, gs = k / groups;
-    const int r0 = (blockIdx.y * DQ_WARPS + warp) * DQ_ROWS;
+    const int r0 = ((blockIdx.z * gridDim.y + blockIdx.y) * DQ_WARPS + warp) * DQ_ROWS;
+    if (r0 >= kp) return;                                         // whole warps
     PairConst<BITS, T> pc[4];
     int g_have = -1;
 #pragma unroll
@@ -117,8 +118,8 @@ dequant_kernel(const uint32_t* __restrict__ qweight, const int32_t* __restrict__
         // the groups of the 4 packed rows: one value of k per lane
         int gl = 0;
         {
-            const int kk = (r0 + rb) * PACK + lane;
-            if (lane < 4 * PACK && kk < k) gl = g_idx ? min(max(__ldg(g_idx + kk), 0), groups - 1) : kk / gs;
+            const unsigned kk = unsigned(r0 + rb) * PACK + lane;
+            if (lane < 4 * PACK && kk < unsigned(k)) gl = g_idx ? min(max(__ldg(g_idx + kk), 0), groups - 1) : int(kk) / gs;
         }
         const unsigned mixed = __ballot_sync(0xffffffffu, gl != __shfl_sync(0xffffffffu, gl, lane & ~(PACK - 1)));
 #pragma unroll
@@ -232,8 +233,8 @@ int launch_dequant_pitch(cudaStream_t st, const uint32_t* qweight, const int32_t
                          const void* scales, void* w_out, int n, int k, int groups, int bits, int dtype, long long pitch) {
     const int pack = 32 / bits;
     if (n == 0 || k == 0) return MT_OK;
-    const dim3 grid((n + 255) / 256, (k / pack + DQ_WARPS * DQ_ROWS - 1) / (DQ_WARPS * DQ_ROWS));
-    if (grid.y > 65535) return MT_ERR_TOO_LARGE;
+    const unsigned runs = (unsigned)((k / pack + DQ_WARPS * DQ_ROWS - 1) / (DQ_WARPS * DQ_ROWS)), ny = runs < 65535u ? runs : 65535u;
+    const dim3 grid((n + 255) / 256, ny, (runs + ny - 1) / ny);
 #define MT_DQ(B, TT) dequant_kernel<B, TT><<<grid, DQ_WARPS * 32, 0, st>>>(qweight, g_idx, qzeros, \
         reinterpret_cast<const TT*>(scales), reinterpret_cast<TT*>(w_out), n, k, groups, pitch)
     if (bits == 4) { if (dtype == MT_F16) MT_DQ(4, __half); else MT_DQ(4, __nv_bfloat16); }

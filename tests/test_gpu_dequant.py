@@ -102,3 +102,20 @@ def test_dequant_ragged_shapes_are_bit_exact(M, bits, dtype, k, n, gs, act):
     ref = O.dequantize_packed(c["qweight"], g_idx, c["qzeros"], c["scales"], bits)
     w = dequantize_packed(c["qweight"].to(DEV), g_idx.to(DEV) if act else None, c["qzeros"].to(DEV), c["scales"].to(DEV), bits)
     assert torch.equal(w.cpu().view(torch.int16), ref.view(torch.int16))
+
+
+@pytest.mark.parametrize("bits,k", [(4, (1 << 24) + 512), (8, (1 << 23) + 384)])
+def test_dequant_of_more_rows_than_one_grid_dimension(M, bits, k):
+    """A tall, narrow weight: more runs of packed rows than the grid's second dimension holds."""
+    from minit_b200.quantize.tensor import dequantize_packed
+    n, gs, pack = 8, 128, 32 // bits
+    gen = torch.Generator(device=DEV).manual_seed(bits)
+    words = lambda *shape: torch.randint(-2 ** 31, 2 ** 31, shape, dtype=torch.int64, device=DEV, generator=gen).to(torch.int32)
+    qw, qz = words(k // pack, n), words(k // gs, n // pack)
+    s = (0.002 + 0.018 * torch.rand((k // gs, n), device=DEV, generator=gen)).half()
+    w = dequantize_packed(qw, None, qz, s, bits)
+    edge = 65535 * 32 * pack
+    for k0 in (0, edge - 256, edge, k - 256):
+        g0, rows = k0 // gs, slice(k0 // pack, k0 // pack + 256 // pack)
+        ref = O.dequantize_packed(qw[rows].cpu(), None, qz[g0:g0 + 2].cpu(), s[g0:g0 + 2].cpu(), bits)
+        assert torch.equal(w[k0:k0 + 256].cpu().view(torch.int16), ref.view(torch.int16)), k0
