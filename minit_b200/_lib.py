@@ -21,7 +21,15 @@ if not os.path.exists(LIB_PATH):
 
 lib = ctypes.CDLL(LIB_PATH)
 
-from . import _host  # noqa: E402  (linked against libminit_b200.so beside it)
+try:
+    from . import _host  # noqa: E402  (linked against libminit_b200.so beside it)
+    _built_for = _host.torch_version
+except (ImportError, AttributeError) as e:
+    raise ImportError(f"the host-call extension minit_b200/_host*.so is missing or does not load in this Python ({e}): build it with "
+                      "`python minit_b200/csrc/build.py` (needs g++ and torch's headers)") from e
+if _built_for != torch.__version__:
+    raise ImportError(f"minit_b200/_host*.so was built for torch {_built_for}, this is {torch.__version__}: build it again with "
+                      "`python minit_b200/csrc/build.py`")
 
 MT_F16, MT_BF16 = 0, 1
 FLAG_FORCE_SMALL, FLAG_FORCE_TC, FLAG_PDL, FLAG_FORCE_VEC, FLAG_FORCE_UMMA, FLAG_AR_SHORT_WAIT, FLAG_FORCE_MID = 1, 2, 4, 16, 32, 64, 128

@@ -6,11 +6,13 @@
 does not import the minit_b200 package, whose import binds the library's symbols)
 
 Objects go to minit_b200/csrc/_obj/, the library to minit_b200/libminit_b200.so and the host-call extension (host.cc, built
-with g++ against torch's headers) to minit_b200/_host.so (in-tree, so they travel with the source tree; all are
-git-ignored).  A source is recompiled when it or any header is newer than its object.
+with g++ against torch's headers) to minit_b200/_host<ABI tag>.so (in-tree, so they travel with the source tree; all are
+git-ignored).  A source is recompiled when it or any header is newer than its object; the extension also when it was built
+for another torch.
 """
 from __future__ import annotations
 
+import importlib.metadata
 import importlib.util
 import os
 import shutil
@@ -23,7 +25,8 @@ CSRC = os.path.dirname(os.path.abspath(__file__))
 HERE = os.path.dirname(CSRC)
 OBJ = os.path.join(CSRC, "_obj")
 LIB = os.path.join(HERE, "libminit_b200.so")
-HOST = os.path.join(HERE, "_host.so")
+HOST = os.path.join(HERE, "_host" + sysconfig.get_config_var("EXT_SUFFIX"))       # one Python's ABI, in its name
+HOST_LOG = os.path.join(OBJ, "_host.torch")        # the torch that it was built for
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-Xptxas", "-v"]
@@ -89,21 +92,38 @@ def build(force: bool = False, verbose: bool = False) -> str:
     return LIB
 
 
-def _build_host(force: bool, verbose: bool) -> None:
-    src = os.path.join(CSRC, "host.cc")
-    deps = [src, os.path.join(HERE, "..", "include", "minit_b200.h"), os.path.abspath(__file__)]
-    if not force and os.path.exists(HOST) and os.path.getmtime(HOST) >= max(os.path.getmtime(d) for d in deps):
-        return
+def torch_version() -> str:
+    return importlib.metadata.version("torch")
+
+
+def host_command() -> list:
     torch_dir = os.path.dirname(importlib.util.find_spec("torch").origin)
     cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
     lib = os.path.join(torch_dir, "lib")
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", src, "-o", HOST, "-I" + os.path.join(torch_dir, "include"),
-           "-I" + os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"), "-I" + os.path.join(cuda, "include"),
-           "-I" + sysconfig.get_paths()["include"], "-L" + lib, "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_python",
-           "-L" + HERE, "-l:libminit_b200.so", "-Wl,-rpath,$ORIGIN"]
+    return ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", os.path.join(CSRC, "host.cc"), "-o", HOST,
+            f'-DMT_TORCH_VERSION="{torch_version()}"', "-I" + os.path.join(torch_dir, "include"),
+            "-I" + os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"), "-I" + os.path.join(cuda, "include"),
+            "-I" + sysconfig.get_paths()["include"], "-L" + lib, "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_python",
+            "-L" + HERE, "-l:libminit_b200.so", "-Wl,-rpath,$ORIGIN"]
+
+
+def host_is_current() -> bool:
+    deps = [os.path.join(CSRC, "host.cc"), os.path.join(HERE, "..", "include", "minit_b200.h"), os.path.abspath(__file__)]
+    if not os.path.exists(HOST) or not os.path.exists(HOST_LOG) or os.path.getmtime(HOST) < max(os.path.getmtime(d) for d in deps):
+        return False
+    with open(HOST_LOG) as f:
+        return f.read() == torch_version()
+
+
+def _build_host(force: bool, verbose: bool) -> None:
+    if not force and host_is_current():
+        return
+    cmd = host_command()
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("g++ failed for host.cc:\n" + r.stderr[-4000:])
+    with open(HOST_LOG, "w") as f:
+        f.write(torch_version())
     if verbose:
         print("compiled", HOST)
 
