@@ -182,8 +182,6 @@ inline ArParams make_ar_params(const QGemmArgs& a) {
 
 int launch_dequant(cudaStream_t st, const uint32_t* qweight, const int32_t* g_idx, const uint32_t* qzeros,
                    const void* scales, void* w_out, int n, int k, int groups, int bits, int dtype);
-int launch_dequant_pitch(cudaStream_t st, const uint32_t* qweight, const int32_t* g_idx, const uint32_t* qzeros,     // rows of w_out `pitch` values apart
-                         const void* scales, void* w_out, int n, int k, int groups, int bits, int dtype, long long pitch);
 int launch_dequant_unpacked(cudaStream_t st, const uint8_t* q, const int32_t* g_idx, const uint8_t* z, const void* scales,
                             void* w_out, int n, int k, int groups, int dtype);
 int launch_w8_pack(cudaStream_t st, const int8_t* w, uint32_t* out, int n, int k);
