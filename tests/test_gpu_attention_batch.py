@@ -256,3 +256,35 @@ def test_offsets_past_the_capacity(D, m, d):
     out = D.attention(q, k - 3.0, v, offsets=torch.tensor(offs, dtype=torch.int32, device=DEV))
     clamped = torch.cat([exact(q[s:s + 1, i:i + 1], k[s:s + 1] - 3.0, v[s:s + 1], [min(offs[s] + i, 100)]) for s in range(3) for i in range(m)], dim=1)
     same(out.view(1, 3 * m, -1), clamped, torch.float16)
+
+
+# ---- routes that plain calls do not take --------------------------------------------------------------------------------
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("m,hq,hkv,d", [(1, 8, 2, 128), (2, 8, 1, 64), (4, 4, 4, 128)])
+def test_call_without_a_workspace(D, dtype, m, hq, hkv, d):
+    """mt_attention, and mt_attention_batch with less than it asks for: up to 16 rows on the tile kernel."""
+    from minit_b200 import _lib
+    q, k, v, offs = inputs(3, m, hq, hkv, d, [130, 0, 63], dtype, seed=41)
+    ref = exact(q, k, v, [130, 0, 63])
+    for name, extra in (("mt_attention", ()), ("mt_attention_batch", (None, 0)), ("mt_attention_batch", (torch.zeros(4096, dtype=torch.uint8, device=DEV).data_ptr(), 4096))):
+        out = torch.empty((3, m, hq * d), dtype=dtype, device=DEV)
+        rc = getattr(_lib.lib, name)(_lib.current_stream(q.device), q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), offs.data_ptr(),
+                                     3, m, hq, hkv, d, 0, k.shape[1], 1.0 / math.sqrt(d), *extra, _lib.dtype_code(dtype))
+        assert rc == 0
+        same(out, ref, dtype)
+
+
+@pytest.mark.parametrize("m", [1, 3])
+def test_more_pairs_than_counters(D, m):
+    """2049 sequences of 8 kv heads: whole (sequence, head) pairs per CTA, none of them cut."""
+    b, hq, hkv, d, cap = 2049, 16, 8, 64, 70
+    gen = torch.Generator(device=DEV).manual_seed(m)
+    make = lambda *shape: torch.randn(shape, device=DEV, generator=gen).half()
+    q, k, v = make(b, m, hq, d), make(b, cap, hkv, d), make(b, cap, hkv, d)
+    lengths = torch.randint(0, cap - m + 1, (b,), device=DEV, generator=gen, dtype=torch.int32)
+    out = D.attention(q, k, v, offsets=lengths).view(b, m, hq, d)
+    s = torch.einsum("bmhgd,bthd->bmhgt", q.double().view(b, m, hkv, 2, d), k.double()) / math.sqrt(d)
+    t = torch.arange(cap, device=DEV)
+    seen = t.view(1, 1, cap) <= (lengths.view(b, 1, 1) + torch.arange(m, device=DEV).view(1, m, 1))
+    p = torch.softmax(s.masked_fill(~seen[:, :, None, None, :], -math.inf), dim=-1)
+    same(out, torch.einsum("bmhgt,bthd->bmhgd", p, v.double()).reshape(b, m, hq, d), torch.float16)
