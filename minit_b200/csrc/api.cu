@@ -264,7 +264,8 @@ int mt_unpack(void* stream, const uint32_t* packed, uint8_t* out, int rows, int 
 
 // Where the integer tensor-core kernel beats the register-ring kernel, from timings of both on the linears of a
 // 70B decoder layer split 1, 2, 4 and 8 ways (K or N from 1024 to 57344): the more rows, the smaller the weights at
-// which its set-up is paid back; with few k-blocks (K < 3072) the ring kernel always wins.
+// which its set-up is paid back.  With few k-blocks (K < 3072) it never is; up to 16 rows the ring kernel takes those, from 17
+// the tensor-memory kernel does (mt_qgemm below).
 static bool mid_preferred(int m, int n, int k) {
     if (m < 3 || m > 32 || k < 3072) return false;
     const long long weights = (long long)k * n;

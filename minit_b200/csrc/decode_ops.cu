@@ -501,7 +501,8 @@ int launch_attention_decode(cudaStream_t st, const void* q, const void* k_cache,
 }
 
 // ----------------------------------------------------------------------------------------------
-// Attention for prefill-sized and multi-sequence batches, any head size that is a multiple of 32 up to 256:
+// Attention for prefill-sized and multi-sequence batches, any head size that is a multiple of 32 up to 256 (heads of 64 and 128
+// come here only with a scale that is not above zero: attention.cu has tensor-core kernels for them):
 //   out[b, i, n, :] = softmax_t(q[b, i, n, :] . k[b, t, n / group, :] * scale, t <= offset_b + i) @ v[b, :, n / group, :]
 // (examples/llama3_70b.py:103-115: scores for every (query, key) pair, -inf above the diagonal shifted by the cached
 // positions, softmax over the keys, weighted sum of the values).  One warp per (sequence, head, four query positions): a

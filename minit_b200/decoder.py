@@ -221,7 +221,7 @@ class QAttention(Module):
         m = x.shape[0]
         if self.head_size == 128 and self.nr_querys // self.nr_kv <= 8 and m <= 16:
             a = attention_decode(q, cache, offset)                 # split over the cached positions: the decode kernel
-        else:                                                      # prefill-sized inputs and other head sizes: one warp per query row
+        else:                                                      # prefill-sized inputs and other head sizes: the batch kernels
             a = attention(q.unsqueeze(0), cache.k.unsqueeze(0), cache.v.unsqueeze(0), offset).view(m, -1)
         cache.length = max(cache.length, offset + m)
         o = self.o_proj
