@@ -89,11 +89,12 @@ constexpr int DQ_WARPS = 4, DQ_ROWS = 8;         // packed rows per warp: 64 (32
 
 }  // namespace
 
-// grid: (256-column windows, runs of DQ_WARPS * DQ_ROWS packed rows over y and z).  `pitch` is n in an argument of its own: with row
-// addresses formed from n the kernel takes 31.3 us where it takes 29.3 (4096 x 14336).  A packed row whose
+// grid: (256-column windows, runs of DQ_WARPS * DQ_ROWS packed rows); TALL: more runs than the grid's y holds, over y and z, in an
+// instance of its own (in one kernel for both, a first pass on cold memory took 50.3 us where it takes 46.3: 4096 x 14336).
+// `pitch` is n in an argument of its own: with row addresses formed from n the kernel takes 31.3 us, 29.3 as it is.  A packed row whose
 // values of k all belong to one group (contiguous groups, or a g_idx that is) uses one set of constants per group; a mixed
 // row (act-order) fetches the constants of every k: a block's window of scales and zeros (20 KB for 32 groups) stays in L1.
-template <int BITS, typename T>
+template <int BITS, typename T, bool TALL>
 __global__ void __launch_bounds__(DQ_WARPS * 32)
 dequant_kernel(const uint32_t* __restrict__ qweight, const int32_t* __restrict__ g_idx,
                const uint32_t* __restrict__ qzeros, const T* __restrict__ scales,
@@ -103,8 +104,8 @@ dequant_kernel(const uint32_t* __restrict__ qweight, const int32_t* __restrict__
     const bool live = (blockIdx.x * 32 + lane) * 8 < n;           // lanes past the last column stay for the warp's shuffles
     const int c = live ? (blockIdx.x * 32 + lane) * 8 : 0;
     const int kp = k / PACK, gs = k / groups;
-    const int r0 = ((blockIdx.z * gridDim.y + blockIdx.y) * DQ_WARPS + warp) * DQ_ROWS;
-    if (r0 >= kp) return;                                         // whole warps
+    const int r0 = ((TALL ? blockIdx.z * gridDim.y + blockIdx.y : blockIdx.y) * DQ_WARPS + warp) * DQ_ROWS;
+    if (TALL && r0 >= kp) return;                                 // whole warps
     PairConst<BITS, T> pc[4];
     int g_have = -1;
 #pragma unroll
@@ -119,8 +120,8 @@ dequant_kernel(const uint32_t* __restrict__ qweight, const int32_t* __restrict__
         // the groups of the 4 packed rows: one value of k per lane
         int gl = 0;
         {
-            const unsigned kk = unsigned(r0 + rb) * PACK + lane;
-            if (lane < 4 * PACK && kk < unsigned(k)) gl = g_idx ? min(max(__ldg(g_idx + kk), 0), groups - 1) : int(kk) / gs;
+            const int kk = (r0 + rb) * PACK + lane;               // TALL: past 2^31 it must not come out below k
+            if (lane < 4 * PACK && (TALL ? unsigned(kk) < unsigned(k) : kk < k)) gl = g_idx ? min(max(__ldg(g_idx + kk), 0), groups - 1) : kk / gs;
         }
         const unsigned mixed = __ballot_sync(0xffffffffu, gl != __shfl_sync(0xffffffffu, gl, lane & ~(PACK - 1)));
 #pragma unroll
@@ -236,8 +237,8 @@ int launch_dequant(cudaStream_t st, const uint32_t* qweight, const int32_t* g_id
     if (n == 0 || k == 0) return MT_OK;
     const unsigned runs = (unsigned)((k / pack + DQ_WARPS * DQ_ROWS - 1) / (DQ_WARPS * DQ_ROWS)), ny = runs < 65535u ? runs : 65535u;
     const dim3 grid((n + 255) / 256, ny, (runs + ny - 1) / ny);
-#define MT_DQ(B, TT) dequant_kernel<B, TT><<<grid, DQ_WARPS * 32, 0, st>>>(qweight, g_idx, qzeros, \
-        reinterpret_cast<const TT*>(scales), reinterpret_cast<TT*>(w_out), n, k, groups, n)
+    auto go = [&](auto kern, auto* sc, auto* out) { kern<<<grid, DQ_WARPS * 32, 0, st>>>(qweight, g_idx, qzeros, sc, out, n, k, groups, n); };
+#define MT_DQ(B, TT) go(grid.z > 1 ? dequant_kernel<B, TT, true> : dequant_kernel<B, TT, false>, reinterpret_cast<const TT*>(scales), reinterpret_cast<TT*>(w_out))
     if (bits == 4) { if (dtype == MT_F16) MT_DQ(4, __half); else MT_DQ(4, __nv_bfloat16); }
     else           { if (dtype == MT_F16) MT_DQ(8, __half); else MT_DQ(8, __nv_bfloat16); }
 #undef MT_DQ
