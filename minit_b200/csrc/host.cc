@@ -265,6 +265,31 @@ PyObject* attention_decode(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     });
 }
 
+// (q, k_cache, v_cache, offset, offsets): the scratch is the call's own
+PyObject* attention(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+    return guarded(nargs, 5, [&](Call& c) -> at::Tensor {
+        const int64_t offset = as_long(a[3], c);
+        const at::Tensor *q = c.tensor(a[0]), *kc = c.tensor(a[1]), *vc = c.tensor(a[2]), *offs = c.optional(a[4]);
+        if (!c.ok) return {};
+        c.need(q->dim() == 4 && kc->dim() == 4 && kc->sizes() == vc->sizes() && kc->scalar_type() == q->scalar_type() &&
+               vc->scalar_type() == q->scalar_type() && dtype_code(*q) >= 0 && q->numel() > 0 && kc->numel() > 0);
+        if (!c.ok) return {};
+        const int64_t b = q->size(0), m = q->size(1), hq = q->size(2), d = q->size(3), cap = kc->size(1), hkv = kc->size(2);
+        c.need(kc->size(0) == b && kc->size(3) == d && hq % hkv == 0 && b < INT32_MAX && m < INT32_MAX && hq < INT32_MAX && cap < INT32_MAX && d <= 256);
+        if (offs) c.need(offs->dim() == 1 && offs->size(0) == b && is(*offs, at::kInt));
+        if (!c.ok) return {};
+        const Guard guard(c);
+        at::Tensor out = at::empty({b, m, hq * d}, q->options()), ws;
+        const size_t need = mt_attention_batch_workspace_bytes(m, hq, hkv, d);
+        if (need) ws = at::empty({int64_t(need)}, q->options().dtype(at::kByte));
+        const bool done = launch(c, nullptr, 0, [&](cudaStream_t st, void*, size_t) {
+            return mt_attention_batch(st, ptr(q), ptr(kc), ptr(vc), out.data_ptr(), (const int32_t*)ptr(offs), b, m, hq, hkv, d, offset, cap,
+                                      float(1.0 / std::sqrt(double(d))), need ? ws.data_ptr() : nullptr, need, dtype_code(*q));
+        });
+        return done ? out : at::Tensor();
+    });
+}
+
 // (x, weight, eps)
 PyObject* rms_norm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     return guarded(nargs, 3, [&](Call& c) -> at::Tensor {
@@ -297,7 +322,7 @@ PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
 
 #define MT_FN(f) {#f, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {MT_FN(bind), MT_FN(qgemm), MT_FN(qgemm_ordered), MT_FN(qgemm_residual), MT_FN(qgemm_swiglu), MT_FN(qkv_rope),
-                         MT_FN(attention_decode), MT_FN(rms_norm), {nullptr, nullptr, 0, nullptr}};
+                         MT_FN(attention_decode), MT_FN(attention), MT_FN(rms_norm), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

@@ -142,6 +142,11 @@ def attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, off
     tokens of every sequence already appended at rows offset_b .. offset_b + M - 1; returns [B, M, hq * d].  ``offsets``
     (int32 [B] on the device) gives every sequence its own number of cached positions, else ``offset`` holds for all.
     Any head size that is a multiple of 32 up to 256."""
+    if out is None:
+        y = _lib._host.attention(q, k_cache, v_cache, offset, offsets)
+        if y is not None:
+            _lib.attention_devices.add(y.get_device())
+            return y
     dev = _lib.require_cuda(q, k_cache, v_cache, offsets)
     if q.dim() != 4 or k_cache.dim() != 4 or k_cache.shape != v_cache.shape:
         raise ValueError("q must be [B, M, hq, d] and the caches [B, capacity, hkv, d]")

@@ -126,3 +126,24 @@ def test_graph_capture(lib_built):
         g.replay()
     torch.cuda.synchronize()
     assert torch.equal(y, ref)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("m,hq,hkv,d", [(1, 8, 2, 128), (2, 4, 4, 64), (40, 8, 2, 128), (3, 4, 2, 96)])
+def test_attention_same_bits_as_the_wrapper(lib_built, dtype, m, hq, hkv, d):
+    from minit_b200 import _lib, decoder as D
+    q = torch.randn((3, m, hq, d), device=DEV).to(dtype)
+    k, v = (torch.randn((3, 200, hkv, d), device=DEV).to(dtype) for _ in range(2))
+    offs = torch.tensor([150, 0, 64], dtype=torch.int32, device=DEV)
+    f = _lib._host.attention
+    for args, kw in (((q, k, v, 0, offs), dict(offsets=offs)), ((q, k, v, 100, None), dict(offset=100))):
+        ref = D.attention(q, k, v, out=torch.empty((3, m, hq * d), dtype=dtype, device=DEV), **kw)
+        y = f(*args)
+        assert y.shape == ref.shape and torch.equal(y, ref) and torch.equal(D.attention(q, k, v, **kw), ref)
+    for bad in ((q[0], k, v, 0, None), (q, k[:2], v[:2], 0, None), (q, k, v[:, :100], 0, None), (q, k.float(), v, 0, None), (q, k, v, 0, offs.long()),
+                (q, k, v, 0, offs[:2]), (q, k, v, 200, None), (q, k, v, -1, None), (q, k, v, 0.0, None), (q[:, :0], k, v, 0, None), (q.cpu(), k, v, 0, None),
+                (q, k.transpose(0, 1).contiguous().transpose(0, 1), v, 0, None)):
+        assert f(*bad) is None
+    with pytest.raises(Exception):
+        D.attention(q, k, v, 200)
